@@ -5,6 +5,7 @@
 //  - incident fields of unit-current closed loops and of a plane wave, tested
 //    onto the PWC/PWL basis (the loop right-hand sides).
 #include "green_host.h"
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -13,12 +14,6 @@
 namespace marie {
 
 typedef cplx<double> zd;
-
-struct Rule3 {          // tensor Gauss rule on [-1,1]^3, first variable fastest
-  const double* x;      // np*3
-  const double* w;      // np
-  int np;
-};
 
 // G_N.m entries [-Gyy-Gzz, Gxy, Gxz, -Gxx-Gzz, Gyz, -Gxx-Gyy]
 __device__ __forceinline__ void gn_kernel(double dx, double dy, double dz, double k0, zd* f) {
@@ -61,73 +56,283 @@ __device__ __forceinline__ void gk_kernel(double dx, double dy, double dz, doubl
   f[2] = scale(fac, -dz);
 }
 
-// (l, l') pairs of the 10 PWL moment products, VV_Nop.m:27-28 (0-based)
-__constant__ int c_ind_l[10] = {0, 1, 2, 3, 0, 0, 0, 1, 1, 2};
-__constant__ int c_ind_lp[10] = {0, 1, 2, 3, 1, 2, 3, 2, 3, 3};
+// ---------------------------------------------------------------------------
+// I_V of one voxel offset m is a six-dimensional Gauss sum over the point
+// pairs (r, r') of two voxels, but the kernel sees only r - r', and along one
+// axis the n x n' pairs have few distinct differences: a symmetric n-point
+// rule used on both sides gives the same difference for (i, j) and
+// (n-1-j, n-1-i), so 9 of 16 for the far rule (n = 4) and 33 of 64 for the
+// medium one (n = 8).  The pair weights and the moments (T_l, B_l' linear or
+// constant along the axis) are summed per difference on the host, and the
+// kernel is evaluated at D^3 points instead of (n n')^3: 729 for 4096, 35937
+// for 262144.  The moments are then applied axis by axis: one thread per
+// (x, y) line sums its D kernel values over z with the three z weights, and
+// the CTA's outputs sum the lines with the x and y weights.
+//
+// The sum is also symmetric under axis permutations (a permuted offset holds
+// the same values with components and moments permuted), so only offsets
+// a >= b >= c are computed and written to their (up to six) places.
+//
+// Bound: FP64 arithmetic (two FMAs per clock and SM), almost all of it the
+// D^3 kernel values.  48^3 PWL, N, the whole call with its copy to the host:
+// 405 -> 9.9 ms (with k_near, which took 95 ms of it on the host).
+// ---------------------------------------------------------------------------
+struct AxisRule {
+  const double* d;      // D differences X - X' on [-1, 1] nodes
+  const double* w;      // [4][D]: weights for (T, B) = (1, 1), (x, 1), (1, x), (x, x)
+  int D;
+};
+constexpr int kVvThreads = 128;
+constexpr int kVvLines = 243;     // lines per pass: three offsets of the far rule (3 * 9^2), odd: conflict-free rows
 
-// One CTA per offset.  out[(mx + n1(my + n2 mz)) + nD*(llp + pwx*comp)]
+enum WType { W_CC = 0, W_LC = 1, W_CL = 2, W_LL = 3 };
+// weight type of moment product j (VV_Nop.m:27-28) along axis d (0 x, 1 y, 2 z)
+__host__ __device__ constexpr int pair_l(int j) { return j < 4 ? j : (j < 7 ? 0 : (j < 9 ? 1 : 2)); }
+__host__ __device__ constexpr int pair_lp(int j) { return j < 4 ? j : (j < 7 ? j - 3 : (j == 7 ? 2 : 3)); }
+__host__ __device__ constexpr int pair_of(int l, int lp) {
+  return l == lp ? l : (l == 0 || lp == 0 ? l + lp + 3 : l + lp + 4);
+}
+__host__ __device__ constexpr int pair_type(int j, int d) {
+  return (pair_l(j) == d + 1 ? 1 : 0) + (pair_lp(j) == d + 1 ? 2 : 0);
+}
+// components of the symmetric N tensor: xx, xy, xz, yy, yz, zz
+__host__ __device__ constexpr int comp_of(int p, int q) { return p + q + (p > 0 && q > 0 ? 1 : 0); }
+__host__ __device__ constexpr int comp_p(int c) { return c < 3 ? 0 : (c < 5 ? 1 : 2); }
+__host__ __device__ constexpr int comp_q(int c) { return c < 3 ? c : (c < 5 ? c - 2 : 2); }
+
+// Axis permutation s (of 0..5): destination axis d takes canonical axis perm(s, d).
+__host__ __device__ constexpr int perm_axis(int s, int d) {
+  const int first = s >> 1, r0 = first == 0 ? 1 : 0, r1 = first == 2 ? 1 : 2;
+  return d == 0 ? first : ((d == 1) == ((s & 1) == 0) ? r0 : r1);
+}
+
+// offs: (a, b, c, rule | 8 * permute).  The first nspec blocks take one offset
+// each (medium rule and the near stand-in), the others three offsets of the
+// far rule.  out[(mx + n1(my + n2 mz)) + nD*(llp + pwx*comp)]
 template <int PWX, int NC, bool ISN>
-__global__ void __launch_bounds__(128) k_vv(const int* offs, const int* rule_of, int noff, Rule3 r0o, Rule3 r0s,
-                                            Rule3 r1o, Rule3 r1s, Rule3 r2o, Rule3 r2s, double dx, double k0,
-                                            int n1, int n2, int n3, zd* out) {
-  __shared__ zd red[4][PWX * NC];
-  const int o = blockIdx.x;
-  if (o >= noff) return;
-  const int mx = offs[3 * o], my = offs[3 * o + 1], mz = offs[3 * o + 2];
-  const int rid = rule_of[o];
-  const Rule3 ro = rid == 0 ? r0o : (rid == 1 ? r1o : r2o);
-  const Rule3 rs = rid == 0 ? r0s : (rid == 1 ? r1s : r2s);
+__global__ void __launch_bounds__(kVvThreads) k_vv(const int4* offs, int nspec, int noff, AxisRule r0, AxisRule r1,
+                                                   AxisRule r2, double dx, double k0, int n1, int n2, int n3,
+                                                   double* out) {
+  extern __shared__ __align__(16) double vsm[];
+  constexpr int NZ = PWX == 1 ? 1 : 3;          // z weight types in use: cc, cl, ll
+  constexpr int NA = NZ * NC * 2;
+  constexpr int NOUT = PWX * NC * 2;
+  constexpr int PER = (3 * NOUT + kVvThreads - 1) / kVvThreads;
+  double* A = vsm;                              // [NA][kVvLines]
+  double* wt = A + NA * kVvLines;               // [4][D], then the differences
+  const int b = blockIdx.x;
+  const bool one = b < nspec;
+  const int o0 = one ? b : nspec + 3 * (b - nspec);
+  const int cnt = one ? 1 : min(3, noff - o0);
+  const int rid = offs[o0].w & 7;
+  const AxisRule r = rid == 0 ? r0 : (rid == 1 ? r1 : r2);
+  const int D = r.D, D2 = D * D;
+  double* dd = wt + 4 * D;
   const double h = dx / 2;
-  const double rmx = mx * dx, rmy = my * dx, rmz = mz * dx;
-  zd acc[PWX][NC];
+  for (int i = threadIdx.x; i < 4 * D; i += kVvThreads) wt[i] = r.w[i];
+  for (int i = threadIdx.x; i < D; i += kVvThreads) dd[i] = h * r.d[i];
+  double acc[PER];
 #pragma unroll
-  for (int a = 0; a < PWX; ++a)
+  for (int v = 0; v < PER; ++v) acc[v] = 0;
+  const int total = cnt * D2;
+  for (int base = 0; base < total; base += kVvLines) {
+    const int nl = min(kVvLines, total - base);
+    __syncthreads();
+    for (int t = threadIdx.x; t < nl; t += kVvThreads) {
+      const int o = (base + t) / D2, line = base + t - o * D2;
+      const int iy = line / D, ix = line - iy * D;
+      const int4 m = offs[o0 + o];
+      const double x = m.x * dx + dd[ix], y = m.y * dx + dd[iy], z0 = m.z * dx;
+      zd a[NZ][NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) acc[a][c] = zd{0, 0};
-  const int npair = ro.np * rs.np;
-  for (int p = threadIdx.x; p < npair; p += blockDim.x) {
-    const int io = p % ro.np, is = p / ro.np;
-    const double X = ro.x[3 * io], Y = ro.x[3 * io + 1], Z = ro.x[3 * io + 2];
-    const double Xp = rs.x[3 * is], Yp = rs.x[3 * is + 1], Zp = rs.x[3 * is + 2];
-    const double w = ro.w[io] * rs.w[is];
-    zd f[NC];
-    if (ISN) gn_kernel(rmx + h * (X - Xp), rmy + h * (Y - Yp), rmz + h * (Z - Zp), k0, f);
-    else gk_kernel(rmx + h * (X - Xp), rmy + h * (Y - Yp), rmz + h * (Z - Zp), k0, f);
-    const double T[4] = {1.0, X * 0.5, Y * 0.5, Z * 0.5};
-    const double B[4] = {1.0, Xp * 0.5, Yp * 0.5, Zp * 0.5};
+      for (int q = 0; q < NZ; ++q)
 #pragma unroll
-    for (int a = 0; a < PWX; ++a) {
-      const double tb = w * T[c_ind_l[a]] * B[c_ind_lp[a]];
+        for (int c = 0; c < NC; ++c) a[q][c] = zd{0, 0};
+      for (int iz = 0; iz < D; ++iz) {
+        zd f[NC];
+        if (ISN) gn_kernel(x, y, z0 + dd[iz], k0, f);
+        else gk_kernel(x, y, z0 + dd[iz], k0, f);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        acc[a][c].x += tb * f[c].x;
-        acc[a][c].y += tb * f[c].y;
+        for (int q = 0; q < NZ; ++q) {
+          const double w = wt[(q == 0 ? W_CC : (q == 1 ? W_CL : W_LL)) * D + iz];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            a[q][c].x = fma(w, f[c].x, a[q][c].x);
+            a[q][c].y = fma(w, f[c].y, a[q][c].y);
+          }
+        }
       }
+#pragma unroll
+      for (int q = 0; q < NZ; ++q)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          A[((q * NC + c) * 2 + 0) * kVvLines + t] = a[q][c].x;
+          A[((q * NC + c) * 2 + 1) * kVvLines + t] = a[q][c].y;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < PER; ++v) {
+      const int u = threadIdx.x + v * kVvThreads;
+      if (u >= cnt * NOUT) break;
+      const int o = u / NOUT, e = u - o * NOUT, ri = e & 1, jc = e >> 1, j = jc / NC, c = jc - j * NC;
+      const int zt = pair_type(j, 2);
+      const double* wx = wt + pair_type(j, 0) * D;
+      const double* wy = wt + pair_type(j, 1) * D;
+      const double* row = A + (((zt == W_CC ? 0 : (zt == W_CL ? 1 : 2)) * NC + c) * 2 + ri) * kVvLines;
+      const int lo = max(o * D2 - base, 0), hi = min((o + 1) * D2 - base, nl);
+      double s = acc[v];
+      for (int t = lo; t < hi; ++t) {
+        const int line = base + t - o * D2;
+        const int iy = line / D, ix = line - iy * D;
+        s = fma(wx[ix] * wy[iy], row[t], s);
+      }
+      acc[v] = s;
     }
   }
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int a = 0; a < PWX; ++a)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      zd v = acc[a][c];
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, s);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, s);
-      }
-      if (lane == 0) red[wid][a * NC + c] = v;
-    }
-  __syncthreads();
   const double J = h * h * h * h * h * h;
   const int64_t nD = (int64_t)n1 * n2 * n3;
-  const int64_t g = mx + (int64_t)n1 * (my + (int64_t)n2 * mz);
-  for (int i = threadIdx.x; i < PWX * NC; i += blockDim.x) {
-    zd s = {0, 0};
-    for (int ww = 0; ww < (int)(blockDim.x >> 5); ++ww) s = s + red[ww][i];
-    const int a = i / NC, c = i % NC;
-    out[g + nD * (a + PWX * c)] = scale(s, J);
+#pragma unroll
+  for (int v = 0; v < PER; ++v) {
+    const int u = threadIdx.x + v * kVvThreads;
+    if (u >= cnt * NOUT) break;
+    const int o = u / NOUT, e = u - o * NOUT, ri = e & 1, jc = e >> 1, j = jc / NC, c = jc - j * NC;
+    const int4 m = offs[o0 + o];
+    const int t[3] = {m.x, m.y, m.z};
+    const int np = (m.w & 8) ? 6 : 1;
+    for (int s = 0; s < np; ++s) {
+      const int p0 = perm_axis(s, 0), p1 = perm_axis(s, 1), p2 = perm_axis(s, 2);
+      const int mx = t[p0], my = t[p1], mz = t[p2];
+      if (mx >= n1 || my >= n2 || mz >= n3) continue;
+      bool again = false;          // equal offsets: the first permutation writes the place
+      for (int q = 0; q < s; ++q)
+        again = again || (t[perm_axis(q, 0)] == mx && t[perm_axis(q, 1)] == my && t[perm_axis(q, 2)] == mz);
+      if (again) continue;
+      auto back = [&](int ax) { return p0 == ax ? 0 : (p1 == ax ? 1 : 2); };
+      const int l = pair_l(j), lp = pair_lp(j);
+      const int jj = PWX == 1 ? 0 : pair_of(l ? back(l - 1) + 1 : 0, lp ? back(lp - 1) + 1 : 0);
+      int cc;
+      if (ISN) cc = comp_of(back(comp_p(c)), back(comp_q(c)));
+      else cc = back(c);
+      out[2 * (mx + (int64_t)n1 * (my + (int64_t)n2 * mz) + nD * (jj + PWX * cc)) + ri] = acc[v] * J;
+    }
   }
+}
+
+// The accurate near zone (green_host.h, near_zone_offset) of the offsets
+// {0,1}^3 on the GPU: the same cubature, its points spread over the CTAs
+// (Gauss node i of the first variable, piece and pyramid, offset).  Each CTA
+// leaves the partial sums of its order^2 points; k_near_sum adds the CTAs of
+// an offset in a fixed order.  On the host this took 95 ms of every assembly
+// (one core, 480 thousand points, three kernel values each).
+constexpr int kNearOrder = 16;
+constexpr int kNearThreads = 128;
+
+template <int PWX, int NC, bool ISN>
+__global__ void __launch_bounds__(kNearThreads) k_near(const double* gx, const double* gw, double res, double k0,
+                                                       int n1, int n2, int n3, double* part) {
+  __shared__ double F[kNearThreads][2][2 * NC];   // the two terms' kernel values with the quadrature weight
+  __shared__ double Wm[kNearThreads][2][PWX];     // W_l and W_l - W_l(0)
+  const int m[3] = {(int)(blockIdx.z & 1), (int)(blockIdx.z >> 1 & 1), (int)(blockIdx.z >> 2)};
+  if (m[0] >= n1 || m[1] >= n2 || m[2] >= n3) return;
+  const int i = blockIdx.x, piece = blockIdx.y / 3, e = blockIdx.y - 3 * piece;
+  double L[3], a[3], sg[3];
+  bool corner = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int upper = piece >> (2 - d) & 1;
+    const double lo = m[d] == 0 ? (upper ? 0.0 : -res) : (upper ? res : 0.0);
+    const double hi = m[d] == 0 ? (upper ? res : 0.0) : (upper ? 2 * res : res);
+    a[d] = lo;
+    L[d] = hi - lo;
+    if (!(lo == 0.0 || hi == 0.0)) corner = false;
+    sg[d] = hi > 0.0 ? 1.0 : -1.0;
+  }
+  const double vol = L[0] * L[1] * L[2];
+  auto weights = [&](const double* u, double* W) {
+    double ov[3][4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        ov[d][q] = PWX == 1 && q ? 0.0 : green_host::moment_overlap(u[d], m[d], res, (q & 1) != 0, (q & 2) != 0);
+#pragma unroll
+    for (int j = 0; j < PWX; ++j) W[j] = ov[0][pair_type(j, 0)] * ov[1][pair_type(j, 1)] * ov[2][pair_type(j, 2)];
+  };
+  const double zero[3] = {0.0, 0.0, 0.0};
+  double W0[PWX], W[PWX];
+  weights(zero, W0);
+  const int f = (e + 1) % 3, g = (e + 2) % 3;
+  double acc = 0;
+  const bool run = corner || e == 0;              // pieces away from 0 take one tensor rule
+  for (int base = 0; run && base < kNearOrder * kNearOrder; base += kNearThreads) {
+    const int j = (base + threadIdx.x) / kNearOrder, k = (base + threadIdx.x) - j * kNearOrder;
+    const double wq = gw[i] * gw[j] * gw[k] * vol;
+    zd Kf[NC], Ks[NC], Kt[NC];
+    double u[3], ut[3];
+    double c1 = wq, c2 = 0;
+    if (!corner) {
+      u[0] = a[0] + L[0] * gx[i];
+      u[1] = a[1] + L[1] * gx[j];
+      u[2] = a[2] + L[2] * gx[k];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) ut[d] = u[d];
+    } else {
+      const double t = gx[i];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        ut[d] = sg[d] * L[d] * (d == e ? 1.0 : (d == f ? gx[j] : gx[k]));
+        u[d] = t * ut[d];
+      }
+      c1 = wq * t * t;
+      c2 = ISN ? wq / t : 0.0;
+    }
+    (void)g;
+    if (ISN) gn_kernel(u[0], u[1], u[2], k0, Kf);
+    else gk_kernel(u[0], u[1], u[2], k0, Kf);
+    if (ISN && corner) {
+      gn_kernel(u[0], u[1], u[2], 0.0, Ks);
+      gn_kernel(ut[0], ut[1], ut[2], 0.0, Kt);
+    } else {
+#pragma unroll
+      for (int c = 0; c < NC; ++c) Ks[c] = Kt[c] = zd{0, 0};
+    }
+    weights(u, W);
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      F[threadIdx.x][0][2 * c] = c1 * (Kf[c].x - Ks[c].x);
+      F[threadIdx.x][0][2 * c + 1] = c1 * (Kf[c].y - Ks[c].y);
+      F[threadIdx.x][1][2 * c] = c2 * Kt[c].x;
+      F[threadIdx.x][1][2 * c + 1] = c2 * Kt[c].y;
+    }
+#pragma unroll
+    for (int l = 0; l < PWX; ++l) {
+      Wm[threadIdx.x][0][l] = W[l];
+      Wm[threadIdx.x][1][l] = W[l] - W0[l];
+    }
+    __syncthreads();
+    if (threadIdx.x < PWX * NC * 2) {
+      const int l = threadIdx.x / (2 * NC), q = threadIdx.x - l * 2 * NC;
+      for (int t = 0; t < kNearThreads; ++t)
+        acc += F[t][0][q] * Wm[t][0][l] + F[t][1][q] * Wm[t][1][l];
+    }
+  }
+  if (threadIdx.x < PWX * NC * 2)
+    part[(((int64_t)blockIdx.z * 24 + blockIdx.y) * kNearOrder + i) * (PWX * NC * 2) + threadIdx.x] = acc;
+}
+
+// out at offset blockIdx.x of {0,1}^3: its CTAs' partial sums, in order
+template <int PWX, int NC>
+__global__ void k_near_sum(const double* part, int n1, int n2, int n3, double* out) {
+  const int mx = blockIdx.x & 1, my = blockIdx.x >> 1 & 1, mz = blockIdx.x >> 2;
+  if (mx >= n1 || my >= n2 || mz >= n3 || threadIdx.x >= PWX * NC * 2) return;
+  const int l = threadIdx.x / (2 * NC), q = threadIdx.x - l * 2 * NC, c = q >> 1, ri = q & 1;
+  double s = 0;
+  for (int b = 0; b < 24 * kNearOrder; ++b)
+    s += part[((int64_t)blockIdx.x * 24 * kNearOrder + b) * (PWX * NC * 2) + threadIdx.x];
+  const int64_t nD = (int64_t)n1 * n2 * n3;
+  out[2 * (mx + (int64_t)n1 * (my + (int64_t)n2 * mz) + nD * (l + PWX * c)) + ri] = s;
 }
 
 void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
@@ -165,33 +370,69 @@ void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
 }
 
 struct DevRule {
-  double* x = nullptr;
-  double* w = nullptr;
-  int np = 0;
+  double* mem = nullptr;
+  AxisRule r{};
 };
 
-static marie_status make_rule(int n, DevRule& r, std::vector<void*>& scratch) {
-  std::vector<double> x1, w1;
-  gauss_legendre(n, x1, w1);
-  const int np = n * n * n;
-  std::vector<double> x(3 * np), w(np);
-  for (int k = 0; k < n; ++k)
-    for (int j = 0; j < n; ++j)
-      for (int i = 0; i < n; ++i) {
-        const int p = i + n * (j + n * k);
-        x[3 * p] = x1[i];
-        x[3 * p + 1] = x1[j];
-        x[3 * p + 2] = x1[k];
-        w[p] = w1[i] * w1[j] * w1[k];
+// Differences and weights of an no x ns point rule along one axis (see k_vv).
+static marie_status make_rule(int no, int ns, DevRule& dr, std::vector<void*>& scratch) {
+  std::vector<double> xo, wo, xs, ws;
+  gauss_legendre(no, xo, wo);
+  gauss_legendre(ns, xs, ws);
+  std::vector<double> d, w[4];
+  std::vector<int> at((size_t)no * ns, -1);
+  for (int i = 0; i < no; ++i)
+    for (int j = 0; j < ns; ++j) {
+      int k = -1;
+      if (no == ns) {            // the same difference: i = j, and (no-1-j, no-1-i)
+        if (i == j && i > 0) k = at[0];
+        else if (i != j) k = at[(size_t)(no - 1 - j) * ns + (no - 1 - i)];
       }
-  if (cudaMalloc(&r.x, x.size() * sizeof(double)) != cudaSuccess) return MARIE_ERR_OOM;
-  scratch.push_back(r.x);
-  if (cudaMalloc(&r.w, w.size() * sizeof(double)) != cudaSuccess) return MARIE_ERR_OOM;
-  scratch.push_back(r.w);
-  cudaMemcpy(r.x, x.data(), x.size() * sizeof(double), cudaMemcpyHostToDevice);
-  cudaMemcpy(r.w, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice);
-  r.np = np;
+      if (k < 0) {
+        k = (int)d.size();
+        d.push_back(i == j && no == ns ? 0.0
+                    : no == ns         ? 0.5 * ((xo[i] - xs[j]) + (xo[no - 1 - j] - xs[no - 1 - i]))
+                                       : xo[i] - xs[j]);
+        for (auto& v : w) v.push_back(0.0);
+      }
+      at[(size_t)i * ns + j] = k;
+      const double ww = wo[i] * ws[j];
+      w[W_CC][k] += ww;
+      w[W_LC][k] += ww * (0.5 * xo[i]);
+      w[W_CL][k] += ww * (0.5 * xs[j]);
+      w[W_LL][k] += ww * (0.5 * xo[i]) * (0.5 * xs[j]);
+    }
+  const int D = (int)d.size();
+  for (auto& v : w) d.insert(d.end(), v.begin(), v.end());
+  if (cudaMalloc(&dr.mem, d.size() * sizeof(double)) != cudaSuccess) return MARIE_ERR_OOM;
+  scratch.push_back(dr.mem);
+  cudaMemcpy(dr.mem, d.data(), d.size() * sizeof(double), cudaMemcpyHostToDevice);
+  dr.r = AxisRule{dr.mem, dr.mem + D, D};
   return MARIE_OK;
+}
+
+template <int PWX, int NC, bool ISN>
+static cudaError_t run_vv(const int4* offs, int nspec, int noff, const DevRule* rules, bool near_exact,
+                          const double* gauss, double* part, double dx, double k0, int n1, int n2, int n3,
+                          double* out) {
+  constexpr int NZ = PWX == 1 ? 1 : 3;
+  int D = 0;
+  for (int i = 0; i < 3; ++i) D = std::max(D, rules[i].r.D);
+  const size_t smem = ((size_t)NZ * NC * 2 * kVvLines + 5 * (size_t)D) * sizeof(double);
+  static std::atomic<uint64_t> done{0};
+  smem_opt_in_device((const void*)k_vv<PWX, NC, ISN>, done);
+  if (near_exact) {
+    k_near<PWX, NC, ISN><<<dim3(kNearOrder, 24, 8), kNearThreads>>>(gauss, gauss + kNearOrder, dx, k0, n1, n2, n3, part);
+    k_near_sum<PWX, NC><<<8, kNearThreads>>>(part, n1, n2, n3, out);
+    g_launches += 2;
+  }
+  const int blocks = nspec + (noff - nspec + 2) / 3;
+  if (blocks > 0) {
+    k_vv<PWX, NC, ISN><<<blocks, kVvThreads, smem>>>(offs, nspec, noff, rules[0].r, rules[1].r, rules[2].r, dx, k0, n1,
+                                                     n2, n3, out);
+    g_launches++;
+  }
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -289,26 +530,8 @@ __global__ void k_plane(const int64_t* idxS, int64_t Ns, int n1, int n2, double 
 
 using namespace marie;
 
-extern "C" marie_status marie_assemble_green_ex(int32_t n1, int32_t n2, int32_t n3, double res, double freq,
-                                                int32_t basis, int32_t kernel, int32_t flags, double* out_host) {
-  if (flags & ~(MARIE_GREEN_SELF_POINT_TERM | MARIE_GREEN_NEAR_EXACT)) {
-    set_error("marie_assemble_green_ex: unknown flags 0x%x", (unsigned)flags);
-    return MARIE_ERR_BAD_ARG;
-  }
-  const marie_status st = marie_assemble_green(n1, n2, n3, res, freq, basis, kernel, out_host);
-  if (st != MARIE_OK) return st;
-  const int pwx = basis == MARIE_PWL ? 10 : 1;
-  if (flags & MARIE_GREEN_NEAR_EXACT) {
-    const double k0 = 2 * M_PI / (299792458.0 / freq);
-    green_host::near_zone_exact(out_host, n1, n2, n3, res, k0, pwx, kernel == 0);
-  } else if ((flags & MARIE_GREEN_SELF_POINT_TERM) && kernel == 0) {
-    green_host::add_self_point_term(out_host, (int64_t)n1 * n2 * n3, pwx, res);
-  }
-  return MARIE_OK;
-}
-
-extern "C" marie_status marie_assemble_green(int32_t n1, int32_t n2, int32_t n3, double res, double freq,
-                                             int32_t basis, int32_t kernel, double* out_host) {
+static marie_status assemble(int32_t n1, int32_t n2, int32_t n3, double res, double freq, int32_t basis,
+                             int32_t kernel, bool near_exact, double* out_host) {
   if (n1 < 1 || n2 < 1 || n3 < 1 || !(res > 0) || !(freq > 0) || !out_host || (basis != 0 && basis != 1) ||
       (kernel != 0 && kernel != 1)) {
     set_error("marie_assemble_green: invalid argument");
@@ -322,66 +545,85 @@ extern "C" marie_status marie_assemble_green(int32_t n1, int32_t n2, int32_t n3,
   // rules: 0 far (4^3 x 4^3), 1 medium (8^3 x 8^3 or min(n)), 2 near stand-in (8^3 x 7^3)
   const int thr = isN ? 5 : 2;
   const int Npm = (n1 <= thr || n2 <= thr || n3 <= thr) ? std::min(n1, std::min(n2, n3)) : 8;
-  std::vector<int> offs, rule;
-  offs.reserve(3 * nD);
-  rule.reserve(nD);
-  for (int mz = 0; mz < n3; ++mz)
-    for (int my = 0; my < n2; ++my)
-      for (int mx = 0; mx < n1; ++mx) {
-        offs.push_back(mx);
-        offs.push_back(my);
-        offs.push_back(mz);
-        int r = 0;
-        if (mx < Npm && my < Npm && mz < Npm) r = 1;
-        if (mx < std::min(2, n1) && my < std::min(2, n2) && mz < std::min(2, n3)) r = 2;
-        rule.push_back(r);
+  // canonical offsets a >= b >= c of which some permutation lies in the box;
+  // the long ones (near stand-in, medium) first, one CTA each
+  int ed[3] = {n1, n2, n3};
+  std::sort(ed, ed + 3, [](int p, int q) { return p > q; });
+  std::vector<int4> offs, far_offs;
+  if (!near_exact)
+    for (int z = 0; z < std::min(2, n3); ++z)
+      for (int y = 0; y < std::min(2, n2); ++y)
+        for (int x = 0; x < std::min(2, n1); ++x) offs.push_back(int4{x, y, z, 2});   // unequal rules: no permutations
+  for (int a = 0; a < ed[0]; ++a)
+    for (int b = 0; b < std::min(a + 1, ed[1]); ++b)
+      for (int c = 0; c < std::min(b + 1, ed[2]); ++c) {
+        if (a < 2) continue;                     // {0,1}^3: the near zone
+        if (a < Npm) offs.push_back(int4{a, b, c, 1 | 8});
+        else far_offs.push_back(int4{a, b, c, 0 | 8});
       }
+  const int nspec = (int)offs.size();
+  offs.insert(offs.end(), far_offs.begin(), far_offs.end());
+  if (offs.empty()) offs.push_back(int4{0, 0, 0, 0});
+  const int noff = (int)(nspec + far_offs.size());
   std::vector<void*> scratch;
   auto done = [&](marie_status s) {
     cudaDeviceSynchronize();
     for (void* p : scratch) cudaFree(p);
     return s;
   };
-  DevRule far, med, nearo, nears;
+  DevRule rules[3];
   marie_status st;
-  if ((st = make_rule(4, far, scratch)) != MARIE_OK) return done(st);
-  if ((st = make_rule(Npm, med, scratch)) != MARIE_OK) return done(st);
-  if ((st = make_rule(8, nearo, scratch)) != MARIE_OK) return done(st);
-  if ((st = make_rule(7, nears, scratch)) != MARIE_OK) return done(st);
-  int *d_offs = nullptr, *d_rule = nullptr;
-  zd* d_out = nullptr;
-  if (cudaMalloc(&d_offs, offs.size() * sizeof(int)) != cudaSuccess) return done(MARIE_ERR_OOM);
-  scratch.push_back(d_offs);
-  if (cudaMalloc(&d_rule, rule.size() * sizeof(int)) != cudaSuccess) return done(MARIE_ERR_OOM);
-  scratch.push_back(d_rule);
-  if (cudaMalloc(&d_out, (size_t)nD * pwx * nc * sizeof(zd)) != cudaSuccess) return done(MARIE_ERR_OOM);
-  scratch.push_back(d_out);
-  cudaMemcpy(d_offs, offs.data(), offs.size() * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(d_rule, rule.data(), rule.size() * sizeof(int), cudaMemcpyHostToDevice);
-  Rule3 r0o{far.x, far.w, far.np}, r1o{med.x, med.w, med.np}, r2o{nearo.x, nearo.w, nearo.np};
-  Rule3 r2s{nears.x, nears.w, nears.np};
-  const int noff = (int)nD;
-  // launch in slices to keep each grid modest
-  const int slice = 1 << 20;
-  for (int o0 = 0; o0 < noff; o0 += slice) {
-    const int cnt = std::min(slice, noff - o0);
-    const int* po = d_offs + 3 * (int64_t)o0;
-    const int* pr = d_rule + o0;
-    if (pwl && isN) k_vv<10, 6, true><<<cnt, 128>>>(po, pr, cnt, r0o, r0o, r1o, r1o, r2o, r2s, res, k0, n1, n2, n3, d_out);
-    else if (pwl) k_vv<10, 3, false><<<cnt, 128>>>(po, pr, cnt, r0o, r0o, r1o, r1o, r2o, r2s, res, k0, n1, n2, n3, d_out);
-    else if (isN) k_vv<1, 6, true><<<cnt, 128>>>(po, pr, cnt, r0o, r0o, r1o, r1o, r2o, r2s, res, k0, n1, n2, n3, d_out);
-    else k_vv<1, 3, false><<<cnt, 128>>>(po, pr, cnt, r0o, r0o, r1o, r1o, r2o, r2s, res, k0, n1, n2, n3, d_out);
-    g_launches++;
-    if (cudaGetLastError() != cudaSuccess) {
-      set_error("assembly kernel launch failed");
-      return done(MARIE_ERR_CUDA);
-    }
+  if ((st = make_rule(4, 4, rules[0], scratch)) != MARIE_OK) return done(st);
+  if ((st = make_rule(Npm, Npm, rules[1], scratch)) != MARIE_OK) return done(st);
+  if ((st = make_rule(8, 7, rules[2], scratch)) != MARIE_OK) return done(st);
+  int4* d_offs = nullptr;
+  double *d_out = nullptr, *d_gauss = nullptr, *d_part = nullptr;
+  auto alloc = [&](void** p, size_t bytes) {
+    if (cudaMalloc(p, bytes) != cudaSuccess) return false;
+    scratch.push_back(*p);
+    return true;
+  };
+  if (!alloc((void**)&d_offs, offs.size() * sizeof(int4)) || !alloc((void**)&d_out, (size_t)nD * pwx * nc * sizeof(zd)) ||
+      !alloc((void**)&d_gauss, 2 * kNearOrder * sizeof(double)) ||
+      !alloc((void**)&d_part, (size_t)8 * 24 * kNearOrder * pwx * nc * sizeof(zd)))
+    return done(MARIE_ERR_OOM);
+  std::vector<double> gx, gw;
+  green_host::gauss01(kNearOrder, gx, gw);
+  cudaMemcpy(d_gauss, gx.data(), kNearOrder * sizeof(double), cudaMemcpyHostToDevice);
+  cudaMemcpy(d_gauss + kNearOrder, gw.data(), kNearOrder * sizeof(double), cudaMemcpyHostToDevice);
+  cudaMemcpy(d_offs, offs.data(), offs.size() * sizeof(int4), cudaMemcpyHostToDevice);
+  cudaError_t e;
+  if (pwl && isN) e = run_vv<10, 6, true>(d_offs, nspec, noff, rules, near_exact, d_gauss, d_part, res, k0, n1, n2, n3, d_out);
+  else if (pwl) e = run_vv<10, 3, false>(d_offs, nspec, noff, rules, near_exact, d_gauss, d_part, res, k0, n1, n2, n3, d_out);
+  else if (isN) e = run_vv<1, 6, true>(d_offs, nspec, noff, rules, near_exact, d_gauss, d_part, res, k0, n1, n2, n3, d_out);
+  else e = run_vv<1, 3, false>(d_offs, nspec, noff, rules, near_exact, d_gauss, d_part, res, k0, n1, n2, n3, d_out);
+  if (e != cudaSuccess) {
+    set_error("assembly kernel launch failed");
+    return done(MARIE_ERR_CUDA);
   }
   if (cudaMemcpy(out_host, d_out, (size_t)nD * pwx * nc * sizeof(zd), cudaMemcpyDeviceToHost) != cudaSuccess) {
     set_error("assembly: device error %s", cudaGetErrorString(cudaGetLastError()));
     return done(MARIE_ERR_CUDA);
   }
   return done(MARIE_OK);
+}
+
+extern "C" marie_status marie_assemble_green(int32_t n1, int32_t n2, int32_t n3, double res, double freq,
+                                             int32_t basis, int32_t kernel, double* out_host) {
+  return assemble(n1, n2, n3, res, freq, basis, kernel, false, out_host);
+}
+
+extern "C" marie_status marie_assemble_green_ex(int32_t n1, int32_t n2, int32_t n3, double res, double freq,
+                                                int32_t basis, int32_t kernel, int32_t flags, double* out_host) {
+  if (flags & ~(MARIE_GREEN_SELF_POINT_TERM | MARIE_GREEN_NEAR_EXACT)) {
+    set_error("marie_assemble_green_ex: unknown flags 0x%x", (unsigned)flags);
+    return MARIE_ERR_BAD_ARG;
+  }
+  MARIE_TRY(assemble(n1, n2, n3, res, freq, basis, kernel, (flags & MARIE_GREEN_NEAR_EXACT) != 0, out_host));
+  // the point term of N at the self offset (near_zone_exact holds it too)
+  if (kernel == 0 && flags)
+    green_host::add_self_point_term(out_host, (int64_t)n1 * n2 * n3, basis == MARIE_PWL ? 10 : 1, res);
+  return MARIE_OK;
 }
 
 static marie_status quad_rule(int nq, double** qx, double** qw, std::vector<void*>& scratch) {

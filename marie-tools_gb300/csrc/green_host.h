@@ -8,6 +8,12 @@
 #include <cstdint>
 #include <vector>
 
+#ifdef __CUDACC__
+#define MARIE_HD __host__ __device__
+#else
+#define MARIE_HD
+#endif
+
 namespace marie {
 namespace green_host {
 
@@ -89,9 +95,9 @@ inline void kernel_at(bool isN, double x, double y, double z, double k0, cd* out
 // [m res - res/2, m res + res/2], of t(u + x' - m res) b(x'), where t and b
 // are s/res on the moment's own axis and 1 otherwise (moments [1, x/res,
 // y/res, z/res] of the voxel, VV_Nop.m:18-19).  Exact (quadratic integrand).
-inline double moment_overlap(double u, int m, double res, bool l_axis, bool lp_axis) {
-  const double lo = std::max(-res / 2, m * res - res / 2 - u);
-  const double hi = std::max(lo, std::min(res / 2, m * res + res / 2 - u));
+MARIE_HD inline double moment_overlap(double u, int m, double res, bool l_axis, bool lp_axis) {
+  const double lo = fmax(-res / 2, m * res - res / 2 - u);
+  const double hi = fmax(lo, fmin(res / 2, m * res + res / 2 - u));
   const double a = l_axis ? (u - m * res) / res : 1.0, b = l_axis ? 1.0 / res : 0.0;
   const double c = lp_axis ? 0.0 : 1.0, d = lp_axis ? 1.0 / res : 0.0;
   const double A = a * c, B = a * d + b * c, C = b * d;
