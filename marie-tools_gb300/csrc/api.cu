@@ -276,7 +276,7 @@ static marie_status choose_tiles(marie_vie* h, PrecState<T>& ps) {
 }
 
 struct CallTiles {
-  int R, TY, TXY, TX;
+  int R, TY, TXY, TX, TZY;
 };
 
 static int pow2floor(int v) {
@@ -295,7 +295,29 @@ static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, 
   const int wxy = (sizeof(T) == 4 ? 16 : 8) * (fast ? 2 : 1);   // row-tile width of the x/y passes
   t.TY = std::max(1, std::min(h->n2, wxy / t.R));
   t.TXY = std::max(1, std::min(2 * h->n1, wxy / t.R));
+  t.TZY = 1;
+  if (fast && sizeof(T) == 4) {
+    // slices of a column (xy4c.cuh): W = 32 elements per tile.  On short axes,
+    // where a tile's W*n/16 tasks leave most of 256 threads idle, more, while
+    // three tiles fit an SM and the CTAs make several waves (32 x 16 x 128 PWC,
+    // 22 right-hand sides: the four passes 253 -> 156 us; at 96^3 64 elements
+    // would slow the y pass 207 -> 243 us).  Fewer where 32 make less than a wave.
+    const int nb = (nr + t.R - 1) / t.R;
+    auto tile = [&](int n, int64_t lines) {
+      auto ctas = [&](int w) { return lines * nb * h->C * ((h->n3 * t.R + w - 1) / w); };
+      int w = std::max(wxy, t.R);
+      while (w * (n / 16) < 256 && (size_t)4 * w * (n + 1) * sizeof(cplx<T>) <= 72 * 1024 && w < 128 &&
+             w < h->n3 * t.R && ctas(2 * w) >= 4 * kSms)
+        w *= 2;
+      while (w > std::max(8, t.R) && ctas(w) < kSms) w /= 2;
+      return w / t.R;
+    };
+    t.TY = tile(h->n1, h->n2);
+    t.TZY = tile(h->n2, 2 * (int64_t)h->n1);
+  }
   t.TX = std::max(1, std::min(2 * h->n1, Wz / t.R));
+  // the complex64 PWL z pass shares each Green value among four elements
+  if (fast && sizeof(T) == 4 && h->pwl) t.TX = std::max(t.TX, 4 / t.R);
   if (!fast) {   // generic passes: keep every tile within one CTA's shared memory
     const size_t sz = sizeof(cplx<T>);
     t.TY = std::min(t.TY, generic_tile_cap(h->n1, 1, t.R, sz));
@@ -405,6 +427,9 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
   a.n1 = h->n1;
   a.n2 = h->n2;
   a.n3 = h->n3;
+  a.g1 = h->n1;
+  a.g2 = h->n2;
+  a.g3 = h->n3;
   a.C = h->C;
   a.Ns = h->Ns;
   a.mode = mode;
@@ -445,6 +470,7 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
     a.TY = ct.TY;
     a.TXY = ct.TXY;
     a.TX = ct.TX;
+    a.TZY = ct.TZY;
     a.nrhs = nr;
     a.in = in + (int64_t)r0 * in_rs;
     a.out = out + (int64_t)r0 * out_rs;

@@ -14,7 +14,7 @@ __host__ __device__ constexpr int kz4_stride(int N, int W) { return N + (W >= 16
 __host__ __device__ constexpr int kz4_halfpad(int W) { return W >= 16 ? 0 : 8 / W; }
 
 // Sequence stride of k4_zp (complex64, packed pairs) in 16-byte pairs.
-__host__ __device__ constexpr int kzp_stride(int N, int W) { return N + (W >= 8 ? 1 : 8 / W); }
+__host__ __device__ constexpr int kzp_stride(int N, int W) { return N + (W >= 4 ? 2 : 8 / W); }
 // k4_zf (float-float, 16-byte elements): the same stride and an odd-half pad
 // of 4/W, which put the eight lanes of every quarter-warp of its five phases
 // on distinct 16-byte bank groups (checked by enumerating lane addresses).
@@ -23,14 +23,53 @@ __host__ __device__ constexpr int kzf_halfpad(int W) { return W >= 8 ? 0 : 4 / W
 
 // Shared-memory bytes of the z pass: k4_z (native complex128: twiddles +
 // both halves), k4_zf (float-float: 32-byte twiddle entries + both halves)
-// or k4_zp (complex64: twiddle tables, slice masks, pairs).
+// or k4_zp (complex64: twiddle tables, slice masks, tile elements, pairs).
 template <typename T>
 __host__ inline size_t kz4_smem(int N, int C, int W) {
   const size_t NB = N / 16;
-  if (sizeof(T) == 4) return 560 * NB + 32 + (size_t)C * W * kzp_stride(N, W) * 16;
+  if (sizeof(T) == 4) return 272 * NB + 64 + 544 + (size_t)C * W * kzp_stride(N, W) * 16;
   if (std::is_same<T, ff>::value) return (36 * NB + 2 * (size_t)C * W * kzf_stride(N, W) + kzf_halfpad(W)) * 16;
   const size_t half = (size_t)C * W * kz4_stride(N, W);
   return (N + 2 * half + kz4_halfpad(W)) * sizeof(cplx<T>);
+}
+
+// Outer length of the complex64 z pass' split N = P x Q: the step that touches
+// HBM.  The short one where it has enough values in flight (NB >= 4: 1.08 against
+// 1.15 ms in the z pass at 112^3 PWC and seven right-hand sides), 16 below.
+__host__ __device__ constexpr int zp_outer(int NB) { return NB >= 4 ? NB : 16; }
+// frequency k of place p (row*16 + col) of a column of the pair layout
+__host__ __device__ constexpr int zp_freq(int NB, int p) { return zp_outer(NB) == NB ? (p >> 4) + NB * (p & 15) : p; }
+
+// Tiles of the complex64 z pass (k4_zp): W = TX*R elements are, from the
+// lowest bit up, R right-hand sides, then the x mirror, then the y mirror,
+// then neighbouring columns, as far as W reaches; mirrors that do not fit
+// are tiles of their own.  At most two CTAs per SM, each walking the tiles.
+struct ZpTiles {
+  int lgW, lgR, cols;       // cols: octant columns kx per tile
+  bool mx, my;              // mirrors inside the tile
+  int ncx, nsub, nb;
+  int total;
+};
+__host__ __device__ inline ZpTiles kzp_tiles(int n1, int n2, int W, int R, int nb) {
+  ZpTiles t;
+  t.lgW = t.lgR = 0;
+  while ((1 << t.lgW) < W) ++t.lgW;
+  while ((1 << t.lgR) < R) ++t.lgR;
+  const int extra = t.lgW - t.lgR;
+  t.mx = extra >= 1;
+  t.my = extra >= 2;
+  t.cols = extra > 2 ? 1 << (extra - 2) : 1;
+  t.ncx = (n1 + t.cols) / t.cols;               // ceil((n1 + 1) / cols)
+  t.nb = nb;
+  t.nsub = nb * (t.mx ? 1 : 2) * (t.my ? 1 : 2);
+  t.total = (n2 + 1) * t.ncx * t.nsub;
+  return t;
+}
+constexpr int kSms = 152;
+template <typename T>
+inline unsigned kzp_grid(const MvArgs<T>& a, int nb) {
+  const int tiles = kzp_tiles(a.n1, a.n2, a.TX * a.R, a.R, nb).total;
+  return (unsigned)(tiles < 2 * kSms ? tiles : 2 * kSms);
 }
 
 template <typename T>
@@ -65,12 +104,15 @@ template <typename T>
 marie_status launch_fast_chunk(marie_vie* h, int op, MvArgs<T>& a, int nb, cudaStream_t stream, cudaEvent_t* ev) {
   const int n1 = h->n1, n2 = h->n2, n3 = h->n3, C = h->C;
   const size_t sz = sizeof(cplx<T>);
+  constexpr bool c64 = std::is_same<T, float>::value;
   const size_t smx = (size_t)(n1 + (size_t)2 * a.TY * a.R * (n1 + 1)) * sz;
-  const size_t smy = (size_t)(n2 + (size_t)2 * a.TXY * a.R * (n2 + 1)) * sz;
+  const size_t smy = (size_t)(n2 + (size_t)2 * (c64 ? a.TZY : a.TXY) * a.R * (n2 + 1)) * sz;
   const size_t smz = kz4_smem<T>(n3, C, a.TX * a.R);
-  dim3 gx((n2 + a.TY - 1) / a.TY, n3, nb * C);
-  dim3 gy((2 * n1 + a.TXY - 1) / a.TXY, n3, nb * C);
+  // x: TY rows (complex64: slices) per tile; y: TXY kx of a row (complex64: TZY slices)
+  dim3 gx(c64 ? (a.g3 + a.TY - 1) / a.TY : (a.g2 + a.TY - 1) / a.TY, c64 ? a.g2 : a.g3, nb * C);
+  dim3 gy(c64 ? (a.g3 + a.TZY - 1) / a.TZY : (2 * n1 + a.TXY - 1) / a.TXY, c64 ? 2 * n1 : a.g3, nb * C);
   dim3 gz(nb, (2 * n1 + a.TX - 1) / a.TX, 2 * n2);
+  if constexpr (c64) gz = dim3(kzp_grid(a, nb));
   if (ev) cudaEventRecord(ev[0], stream);
   launch_x_nb<T>(n1 / 16, false, a, gx, smx, stream);
   MARIE_LAUNCH_CHECK();

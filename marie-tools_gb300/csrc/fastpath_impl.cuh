@@ -16,7 +16,15 @@ static void smem_opt_in(KernelFn fn, std::atomic<uint64_t>& done) {
 template <typename T, int NB>
 static void launch_x(bool inv, const MvArgs<T>& a, dim3 g, size_t smem, cudaStream_t s) {
   static std::atomic<uint64_t> of{0}, oi{0};
-  if (!inv) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (!inv) {
+      smem_opt_in(k4c_fwd_x<NB>, of);
+      k4c_fwd_x<NB><<<g, 256, smem, s>>>(a);
+    } else {
+      smem_opt_in(k4c_inv_x<NB>, oi);
+      k4c_inv_x<NB><<<g, 256, smem, s>>>(a);
+    }
+  } else if (!inv) {
     smem_opt_in(k4_fwd_x<T, NB>, of);
     k4_fwd_x<T, NB><<<g, 256, smem, s>>>(a);
   } else {
@@ -28,7 +36,15 @@ static void launch_x(bool inv, const MvArgs<T>& a, dim3 g, size_t smem, cudaStre
 template <typename T, int NB>
 static void launch_y(bool inv, const MvArgs<T>& a, dim3 g, size_t smem, cudaStream_t s) {
   static std::atomic<uint64_t> of{0}, oi{0};
-  if (!inv) {
+  if constexpr (std::is_same<T, float>::value) {
+    if (!inv) {
+      smem_opt_in(k4c_fwd_y<NB>, of);
+      k4c_fwd_y<NB><<<g, 256, smem, s>>>(a);
+    } else {
+      smem_opt_in(k4c_inv_y<NB>, oi);
+      k4c_inv_y<NB><<<g, 256, smem, s>>>(a);
+    }
+  } else if (!inv) {
     smem_opt_in(k4_fwd_y<T, NB>, of);
     k4_fwd_y<T, NB><<<g, 256, smem, s>>>(a);
   } else {

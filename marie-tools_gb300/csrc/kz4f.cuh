@@ -180,8 +180,13 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
   constexpr int NE = OpTab<PWL, OP>::NE;
   const int bu = blockIdx.x;
   if (!bundle_active(a, bu)) return;
-  const int kyp = blockIdx.z, k0 = blockIdx.y * a.TX;
-  const int n1 = a.n1, n2 = a.n2, m1 = 2 * n1, R = a.R;
+  // blockIdx.z walks y in slot order too: mirrored ky run back to back
+  const int n1 = a.n1, n2 = a.n2, g3 = a.g3, m1 = 2 * n1, R = a.R;
+  const int k0 = blockIdx.y * a.TX;
+  bool my;
+  const int kyo = slot_octant(blockIdx.z, n2, my);
+  const int ky = my ? 2 * n2 - kyo : kyo;
+  const int kyp = (ky & 1) * n2 + (ky >> 1);
   const int W = a.TX * R, wl = min(a.TX, m1 - k0) * R;
   const int lgW = 31 - __clz(W);                // W = TX*R is a power of two
   const int S = kzf_stride(N, W);
@@ -204,8 +209,15 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
   };
   __syncthreads();
   const int64_t row = (int64_t)m1 * R;
-  const int64_t cstride = (int64_t)2 * n2 * N * row;
-  cplx<ff>* base = a.S + (int64_t)bu * C * cstride + (int64_t)kyp * N * row + (int64_t)k0 * R;
+  const int64_t cstride = (int64_t)2 * n2 * g3 * row;
+  cplx<ff>* base = a.S + (int64_t)bu * C * cstride + (int64_t)kyp * g3 * row + (int64_t)k0 * R;
+  // x frequency of element e, and its components' sign changes where a
+  // frequency is mirrored (mirror_mask)
+  auto kx_of = [&](int e) {
+    const int kxp = k0 + (e >> a.lgR), alpha = kxp >= n1 ? 1 : 0;
+    return 2 * (kxp - alpha * n1) + alpha;
+  };
+  auto flips_of = [&](int e) { return mirror_flips<PWL>(kx_of(e) > n1, my); };
 
   // forward step 1: task (e, h, b, c), e fastest; half h of the zero-padded
   // 2N-point transform (h = 1: inputs times w_2N^z), 16-point DFT over a of
@@ -214,12 +226,14 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
     const int e = t & (W - 1), r = t >> lgW;
     const int h = r & 1, r2 = r >> 1;
     const int b = r2 % NB, c = r2 / NB;
-    const unsigned live = a.zq ? a.zq[b] : 0xffffu;   // slices z = NB*q + b
+    const unsigned live = a.zq ? a.zq[b] : inside_bits(g3, NB, b);   // slices z = NB*q + b
+    const bool flip = (flips_of(e) >> c) & 1u;
     ffc2 u[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       cplx<ff> val = (e < wl && ((live >> q) & 1u)) ? base[c * cstride + (int64_t)(NB * q + b) * row + e]
                                                     : cplx<ff>{ff(0), ff(0)};
+      if (flip) val = cplx<ff>{-val.x, -val.y};
       if (h) val = val * a.az.tw2[NB * q + b];
       u[q] = to_ffc2(val);
     }
@@ -246,18 +260,16 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
 
   // Green block multiply, one frequency per item (e, g, k): kz = 2k + g sits
   // in half g at zpos(k >> 4, k & 15); its U block values are contiguous in
-  // the full spectrum at ((ky*2n1 + kx)*2N + kz)*U.
+  // the spectrum at ((kyo*(n1+1) + kxo)*2N + kz)*U (octant columns).
   constexpr int U = OpTab<PWL, OP>::L.nblk;
-  const int beta = kyp / n2, ky = 2 * (kyp - beta * n2) + beta;
   for (int i = threadIdx.x; i < 2 * N * W; i += blockDim.x) {
     const int e = i & (W - 1), pp = i >> lgW;
     const int kxp = k0 + (e >> a.lgR);
     if (kxp >= m1) continue;
     const int g = pp / N, k = pp - g * N;
     const int kz = 2 * k + g;
-    const int alpha = kxp >= n1 ? 1 : 0;
-    const int kx = 2 * (kxp - alpha * n1) + alpha;
-    const cplx<ff>* gp = a.G + (((int64_t)ky * m1 + kx) * (2 * N) + kz) * U;
+    const int kx = kx_of(e), kxo = kx > n1 ? 2 * n1 - kx : kx;
+    const cplx<ff>* gp = a.G + (((int64_t)kyo * (n1 + 1) + kxo) * (2 * N) + kz) * U;
     ffc2* v = buf + g * H + e * S + zpos(k >> 4, k & 15);
     if constexpr (PWL) zpoint_pwl_ff<OP>(v, W * S, gp);
     else zpoint_pwc_ff<OP>(std::make_integer_sequence<int, NE>{}, v, W * S, gp);
@@ -302,14 +314,15 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
       for (int q = 0; q < 16; ++q) u[q] = mulc(u[q], a.az.tw2[NB * q + b]);
     }
     const bool st = act && e < wl;
-    const unsigned live = (a.zq ? a.zq[b] : 0xffffu) >> (8 * h);   // slices z = NB*(8h + j) + b
+    const bool flip = (flips_of(e) >> c) & 1u;
+    const unsigned live = (a.zq ? a.zq[b] : inside_bits(g3, NB, b)) >> (8 * h);   // slices z = NB*(8h + j) + b
     cplx<ff>* dst = base + c * cstride + (int64_t)(NB * 8 * h + b) * row + e;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const cplx<ff> send = h ? u[j] : u[8 + j];
       const cplx<ff> recv = shfl_xor_c(send, W);
       const cplx<ff> out = h ? recv + u[8 + j] : u[j] + recv;
-      if (st && ((live >> j) & 1u)) dst[(int64_t)NB * j * row] = out;
+      if (st && ((live >> j) & 1u)) dst[(int64_t)NB * j * row] = flip ? cplx<ff>{-out.x, -out.y} : out;
     }
   }
 }

@@ -66,6 +66,7 @@ struct BlockTab {
 template <typename T>
 struct MvArgs {
   int n1, n2, n3, C;
+  int g1, g2, g3;             // the caller's grid (four-step passes: g <= n, the transforms pad to n)
   int R;                      // right-hand sides per bundle (interleaved innermost)
   int lgR;                    // log2(R) (R is a power of two)
   int nrhs;                   // right-hand sides in this launch (<= nbundle * R)
@@ -85,7 +86,7 @@ struct MvArgs {
   cplx<T> efac;               // 1/ce (MV_EFIELD)
   const cplx<typename IoOf<T>::type>* addend;   // added to the body output (same strides; may be null)
   // Body occupancy for the pruned four-step passes (null: every row live).
-  // row_live[z*n2 + y]: the grid row (y, z) holds a body voxel; z_live[z]:
+  // row_live[z*g2 + y]: the grid row (y, z) holds a body voxel; z_live[z]:
   // slice z does.  Rows and slices that are not live are zero on input and
   // not needed on output, so the passes neither transform nor store them.
   const unsigned char* row_live;
@@ -96,6 +97,7 @@ struct MvArgs {
   const uint16_t* rowq;
   const uint16_t* zq;
   int TY, TXY, TX;            // tile sizes of the X, Y, Z passes
+  int TZY;                    // slices per tile of the complex64 four-step Y passes
 };
 
 template <typename T>
@@ -110,12 +112,48 @@ __device__ __forceinline__ bool lane_active(const MvArgs<T>& a, int rhs) {
 
 template <typename T>
 __device__ __forceinline__ bool row_is_live(const MvArgs<T>& a, int y, int z) {
-  return a.row_live == nullptr || a.row_live[z * a.n2 + y] != 0;
+  return a.row_live == nullptr || a.row_live[z * a.g2 + y] != 0;
 }
 
 template <typename T>
 __device__ __forceinline__ bool z_is_live(const MvArgs<T>& a, int z) {
   return a.z_live == nullptr || a.z_live[z] != 0;
+}
+
+// Live bits of the four-step index order without a body: bit q of step b is
+// position NB*q + b, live when inside the caller's edge g.
+__device__ __forceinline__ unsigned inside_bits(int g, int NB, int b) {
+  const int cnt = g > b ? (g - b + NB - 1) / NB : 0;   // q with NB*q + b < g
+  return (1u << (cnt < 16 ? cnt : 16)) - 1u;
+}
+
+// The z passes of complex128 walk the y frequencies in slots, a frequency
+// beside its mirror 2n - k: slot 2k and 2k + 1 for 0 < k < n, and the two
+// self-mirror frequencies 0 and n in slots 0 and 1.
+// slot -> octant frequency (0..n) and whether it is the mirrored one
+__device__ __forceinline__ int slot_octant(int slot, int n, bool& mirror) {
+  mirror = slot >= 2 && (slot & 1);
+  return slot == 1 ? n : slot >> 1;
+}
+
+// The Green's tensor at a mirrored frequency is D G D with D = diag(+-1): a
+// mirror along axis d flips the vector components p = d and the linear
+// moments along d (the mirror signs of assembly_fft_circ_tucker_pwl.m:36-47
+// are products of the two components' and the two moments' signs; for K the
+// product carries one more sign, its kernel being odd).  Bit c of the mask:
+// component c changes sign.
+template <bool PWL>
+__host__ __device__ constexpr unsigned mirror_mask(int axis) {
+  unsigned m = 0;
+  for (int c = 0; c < (PWL ? 12 : 3); ++c) {
+    const bool f = PWL ? ((c / 4 == axis) != (c % 4 == axis + 1)) : c == axis;
+    if (f) m |= 1u << c;
+  }
+  return m;
+}
+template <bool PWL>
+__device__ __forceinline__ unsigned mirror_flips(bool mx, bool my) {
+  return (mx ? mirror_mask<PWL>(0) : 0u) ^ (my ? mirror_mask<PWL>(1) : 0u);
 }
 
 // Body-vector output of the modes other than MV_GRID for component c, body

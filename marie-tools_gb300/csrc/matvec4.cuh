@@ -10,7 +10,9 @@
 // makes one shared-memory round trip (the z pass four: forward, multiply,
 // inverse), and every index is a shift or a multiply by a constant.
 // Spectra are kept in natural frequency order: position k of half alpha holds
-// frequency 2k + alpha.  Layouts in HBM are those of matvec.cuh.
+// frequency 2k + alpha.  The x and y passes here serve complex128; complex64 has
+// its own (xy4c.cuh).  Layouts in HBM are those of matvec.cuh over the caller's
+// rows y < g2 and slices z < g3.
 #pragma once
 
 #include "matvec.cuh"
@@ -106,8 +108,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_x(MvArgs<T
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
   if (!bundle_active(a, bu)) return;
   const int z = blockIdx.y, y0 = blockIdx.x * a.TY;
-  const int n2 = a.n2, n3 = a.n3, R = a.R, lgR = a.lgR;
-  const int ty = min(a.TY, n2 - y0);
+  const int g1 = a.g1, g2 = a.g2, g3 = a.g3, R = a.R, lgR = a.lgR;
+  const int ty = min(a.TY, g2 - y0);
   bool any = false;
   for (int yy = 0; yy < ty; ++yy) any = any || row_is_live(a, y0 + yy, z);
   if (!any) return;   // rows without body voxels stay unwritten: the y pass reads them as zero
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_x(MvArgs<T
   cplx<T>* buf = tw + N;
   load_tw(tw, a.ax.tw, N);
   __syncthreads();
-  const int64_t nD = (int64_t)N * n2 * n3;
+  const int64_t nD = (int64_t)g1 * g2 * g3;
   // step 1: task (yy, r, b), b fastest
   for (int t = threadIdx.x; t < ty * R * NB; t += blockDim.x) {
     const int b = t % NB, rr = t / NB;
@@ -124,13 +126,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_x(MvArgs<T
     const int rhs = bu * R + r;
     const bool act = lane_active(a, rhs);
     const auto* in = a.in + (int64_t)rhs * a.in_rs;
-    const int64_t grow = (int64_t)N * (y0 + yy + (int64_t)n2 * z);
+    const int64_t grow = (int64_t)g1 * (y0 + yy + (int64_t)g2 * z);
     cplx<T> v[16], u[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       const int x = NB * q + b;
       cplx<T> val = {0, 0};
-      if (act) {
+      if (act && x < g1) {
         if (a.mode == MV_GRID) {
           val = io_load<T>(in[(int64_t)c * nD + grow + x]);
         } else {
@@ -158,10 +160,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_x(MvArgs<T
   __syncthreads();
   // step 2: task (yy, alpha, k1, r), r fastest; output row [kx' = alpha*N + k][r]
   const int rowlen = 2 * N * R;
-  cplx<T>* dst = a.T1 + (((int64_t)bu * a.C + c) * n3 + z) * (int64_t)n2 * rowlen;
+  cplx<T>* dst = a.T1 + (((int64_t)bu * a.C + c) * g3 + z) * (int64_t)g2 * rowlen;
   for (int t = threadIdx.x; t < ty * 32 * R; t += blockDim.x) {
     const int r = t & (R - 1), q = t >> lgR;
-    const int k1 = q & 15, alpha = (q >> 4) & 1, yy = q >> 5;
+    const int alpha = (q >> 4) & 1, k1 = q & 15, yy = q >> 5;
     if (!row_is_live(a, y0 + yy, z)) continue;
     const cplx<T>* src = buf + ((yy * R + r) * 2 + alpha) * S + k1 * NB;
     cplx<T> w[NB];
@@ -184,8 +186,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
   if (!bundle_active(a, bu)) return;
   const int z = blockIdx.y, y0 = blockIdx.x * a.TY;
-  const int n2 = a.n2, n3 = a.n3, R = a.R, lgR = a.lgR;
-  const int ty = min(a.TY, n2 - y0);
+  const int g1 = a.g1, g2 = a.g2, g3 = a.g3, R = a.R, lgR = a.lgR;
+  const int ty = min(a.TY, g2 - y0);
   bool any = false;
   for (int yy = 0; yy < ty; ++yy) any = any || row_is_live(a, y0 + yy, z);
   if (!any) return;   // no body voxel in these rows: no output
@@ -194,11 +196,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T
   load_tw(tw, a.ax.tw, N);
   __syncthreads();
   const int rowlen = 2 * N * R;
-  const cplx<T>* srow = a.T1 + (((int64_t)bu * a.C + c) * n3 + z) * (int64_t)n2 * rowlen;
+  const cplx<T>* srow = a.T1 + (((int64_t)bu * a.C + c) * g3 + z) * (int64_t)g2 * rowlen;
   // step A: task (yy, alpha, k1, r): inverse NB-point DFT over k2, twiddle
   for (int t = threadIdx.x; t < ty * 32 * R; t += blockDim.x) {
     const int r = t & (R - 1), q = t >> lgR;
-    const int k1 = q & 15, alpha = (q >> 4) & 1, yy = q >> 5;
+    const int alpha = (q >> 4) & 1, k1 = q & 15, yy = q >> 5;
     if (!row_is_live(a, y0 + yy, z)) continue;
     const cplx<T>* in = srow + (int64_t)(y0 + yy) * rowlen + (alpha * N + k1) * R + r;
     cplx<T> w[NB];
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T
   }
   __syncthreads();
   // step B: task (yy, r, b): inverse 16-point DFTs of both halves, combine, epilogue
-  const int64_t nD = (int64_t)N * n2 * n3;
+  const int64_t nD = (int64_t)g1 * g2 * g3;
   for (int t = threadIdx.x; t < ty * R * NB; t += blockDim.x) {
     const int b = t % NB, rr = t / NB;
     const int r = rr & (R - 1), yy = rr >> lgR;
@@ -226,10 +228,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T
     }
     dftn<T, true, 16>(u0);
     dftn<T, true, 16>(u1);
-    const int64_t grow = (int64_t)N * (y0 + yy + (int64_t)n2 * z);
+    const int64_t grow = (int64_t)g1 * (y0 + yy + (int64_t)g2 * z);
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       const int x = NB * q + b;
+      if (x >= g1) break;
       cplx<T> v = u0[q] + mulc(u1[q], a.ax.tw2[x]);
       if (a.mode == MV_GRID) {
         a.out[(int64_t)rhs * a.out_rs + (int64_t)c * nD + grow + x] = io_store(v);
@@ -242,7 +245,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T
 }
 
 // ---------------------------------------------------------------------------
-// Pass Y (forward), n2 = 16*NB.  grid (ceil(2n1/TXY), n3, nbundle*C)
+// Pass Y (forward), n2 = 16*NB.  grid (ceil(2n1/TXY), g3, nbundle*C)
 // buf: sequence s = beta*W + e, stride S, [k1][b]
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_y(MvArgs<T
   if (!bundle_active(a, bu)) return;
   const int z = blockIdx.y, k0 = blockIdx.x * a.TXY;
   if (!z_is_live(a, z)) return;   // slice without body voxels: the z pass reads it as zero
-  const int n1 = a.n1, n3 = a.n3, m1 = 2 * n1, R = a.R;
+  const int g2 = a.g2, g3 = a.g3, m1 = 2 * a.n1, R = a.R;
   const int W = a.TXY * R, wl = min(a.TXY, m1 - k0) * R;
   const int lgW = 31 - __clz(W);   // TXY*R is a power of two
   cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
@@ -261,11 +264,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_y(MvArgs<T
   load_tw(tw, a.ay.tw, N);
   __syncthreads();
   const int64_t row = (int64_t)m1 * R;
-  const cplx<T>* src = a.T1 + (((int64_t)bu * a.C + c) * n3 + z) * (int64_t)N * row + (int64_t)k0 * R;
+  const cplx<T>* src = a.T1 + (((int64_t)bu * a.C + c) * g3 + z) * (int64_t)g2 * row + (int64_t)k0 * R;
   // step 1: task (b, e), e fastest
   for (int t = threadIdx.x; t < W * NB; t += blockDim.x) {
     const int e = t & (W - 1), b = t >> lgW;
-    const unsigned live = a.rowq ? a.rowq[z * 8 + b] : 0xffffu;   // rows y = NB*q + b
+    const unsigned live = a.rowq ? a.rowq[z * 8 + b] : inside_bits(g2, NB, b);   // rows y = NB*q + b
     cplx<T> v[16], u[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
@@ -285,7 +288,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_y(MvArgs<T
   }
   __syncthreads();
   // step 2: task (beta, k1, e), e fastest; S_glob[bu][c][beta*N + k][z][kx'][r]
-  cplx<T>* dst = a.S + ((int64_t)bu * a.C + c) * (int64_t)2 * N * n3 * row + (int64_t)k0 * R;
+  cplx<T>* dst = a.S + ((int64_t)bu * a.C + c) * (int64_t)2 * N * g3 * row + (int64_t)k0 * R;
   for (int t = threadIdx.x; t < 2 * 16 * W; t += blockDim.x) {
     const int e = t & (W - 1), q = t >> lgW;
     const int k1 = q & 15, beta = q >> 4;
@@ -295,7 +298,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_y(MvArgs<T
     dftn<T, false, NB>(w);
     if (e < wl) {
 #pragma unroll
-      for (int k2 = 0; k2 < NB; ++k2) dst[((int64_t)(beta * N + k1 + 16 * k2) * n3 + z) * row + e] = w[k2];
+      for (int k2 = 0; k2 < NB; ++k2) dst[((int64_t)(beta * N + k1 + 16 * k2) * g3 + z) * row + e] = w[k2];
     }
   }
 }
@@ -311,7 +314,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_y(MvArgs<T
   if (!bundle_active(a, bu)) return;
   const int z = blockIdx.y, k0 = blockIdx.x * a.TXY;
   if (!z_is_live(a, z)) return;   // no body voxel in slice z: no output
-  const int n1 = a.n1, n3 = a.n3, m1 = 2 * n1, R = a.R;
+  const int g2 = a.g2, g3 = a.g3, m1 = 2 * a.n1, R = a.R;
   const int W = a.TXY * R, wl = min(a.TXY, m1 - k0) * R;
   const int lgW = 31 - __clz(W);   // TXY*R is a power of two
   cplx<T>* tw = reinterpret_cast<cplx<T>*>(smem_raw);
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_y(MvArgs<T
   load_tw(tw, a.ay.tw, N);
   __syncthreads();
   const int64_t row = (int64_t)m1 * R;
-  const cplx<T>* src = a.S + ((int64_t)bu * a.C + c) * (int64_t)2 * N * n3 * row + (int64_t)k0 * R;
+  const cplx<T>* src = a.S + ((int64_t)bu * a.C + c) * (int64_t)2 * N * g3 * row + (int64_t)k0 * R;
   // step A: task (beta, k1, e)
   for (int t = threadIdx.x; t < 2 * 16 * W; t += blockDim.x) {
     const int e = t & (W - 1), q = t >> lgW;
@@ -327,17 +330,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_y(MvArgs<T
     cplx<T> w[NB];
 #pragma unroll
     for (int k2 = 0; k2 < NB; ++k2)
-      w[k2] = e < wl ? src[((int64_t)(beta * N + k1 + 16 * k2) * n3 + z) * row + e] : cplx<T>{0, 0};
+      w[k2] = e < wl ? src[((int64_t)(beta * N + k1 + 16 * k2) * g3 + z) * row + e] : cplx<T>{0, 0};
     dftn<T, true, NB>(w);
 #pragma unroll
     for (int b = 0; b < NB; ++b) buf[(beta * W + e) * S + k1 * NB + b] = mulc(w[b], tw[b * k1]);
   }
   __syncthreads();
   // step B: task (b, e): inverse 16-point DFTs of both halves, combine, store
-  cplx<T>* dst = a.T1 + (((int64_t)bu * a.C + c) * n3 + z) * (int64_t)N * row + (int64_t)k0 * R;
+  cplx<T>* dst = a.T1 + (((int64_t)bu * a.C + c) * g3 + z) * (int64_t)g2 * row + (int64_t)k0 * R;
   for (int t = threadIdx.x; t < W * NB; t += blockDim.x) {
     const int e = t & (W - 1), b = t >> lgW;
-    const unsigned live = a.rowq ? a.rowq[z * 8 + b] : 0xffffu;   // rows y = NB*q + b
+    const unsigned live = a.rowq ? a.rowq[z * 8 + b] : inside_bits(g2, NB, b);   // rows y = NB*q + b
     cplx<T> u0[16], u1[16];
 #pragma unroll
     for (int k1 = 0; k1 < 16; ++k1) {
@@ -359,5 +362,6 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_y(MvArgs<T
 }  // namespace marie
 
 #include "kz4.cuh"
+#include "xy4c.cuh"
 #include "kz4p.cuh"
 #include "kz4f.cuh"

@@ -11,6 +11,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fastpath.cuh"
 #include "internal.h"
 
 namespace marie {
@@ -98,50 +99,51 @@ __global__ void k_oct_store(const zd* tmp, cplx<T>* dst, int nkx, int nky, int n
   }
 }
 
-// Full spectrum of one block for the four-step z pass, layout
-// [ky][kx][kz][blk] over the whole (2n2, 2n1, 2n3) grid with the circulant
-// mirror signs applied: dst[((ky*2n1 + kx)*2n3 + kz)*U + blk].
+// Spectrum of one block for the four-step z pass, octant columns: for the
+// columns kx in [0, n1], ky in [0, n2] all 2n3 frequencies kz, the z mirror
+// sign applied; the mirrored columns follow by signs of the components
+// (mirror_mask).  dst[((ky*(n1+1) + kx)*2n3 + kz)*U + blk].
 template <typename T>
-__global__ void k_full_store(const zd* tmp, cplx<T>* dst, int n1, int n2, int n3, int U, int blk, int s1, int s2,
-                             int s3, double scl) {
-  const int m1 = 2 * n1, m2 = 2 * n2, m3 = 2 * n3;
+__global__ void k_full_store(const zd* tmp, cplx<T>* dst, int n1, int n2, int n3, int U, int blk, int s3, double scl) {
+  const int m3 = 2 * n3;
   const int nkx = n1 + 1, nky = n2 + 1;
-  const int64_t total = (int64_t)m1 * m2 * m3;
+  const int64_t total = (int64_t)nkx * nky * m3;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int kz = (int)(idx % m3);
     const int64_t r = idx / m3;
-    const int kx = (int)(r % m1);
-    const int ky = (int)(r / m1);
-    const bool mx = kx > n1, my = ky > n2, mz = kz > n3;
-    const int kxo = mx ? m1 - kx : kx, kyo = my ? m2 - ky : ky, kzo = mz ? m3 - kz : kz;
-    const double sg = (double)((mx ? s1 : 1) * (my ? s2 : 1) * (mz ? s3 : 1)) * scl;
-    const zd v = tmp[kxo + (int64_t)nkx * (kyo + (int64_t)nky * kzo)];
+    const int kx = (int)(r % nkx);
+    const int ky = (int)(r / nkx);
+    const bool mz = kz > n3;
+    const double sg = (double)(mz ? s3 : 1) * scl;
+    const zd v = tmp[kx + (int64_t)nkx * (ky + (int64_t)nky * (mz ? m3 - kz : kz))];
     dst[idx * U + blk] = cplx<T>{(T)(v.x * sg), (T)(v.y * sg)};
   }
 }
 
 // The same for the complex64 z pass (k4_zp), pair layout: frequencies 2k and
 // 2k+1 of a column share one 16-byte entry (re, re, im, im) at
-// ((ky*2n1 + kx)*U + blk)*n3 + k.
-__global__ void k_full_store_pair(const zd* tmp, float* dst, int n1, int n2, int n3, int U, int blk, int s1, int s2,
-                                  int s3, double scl) {
-  const int m1 = 2 * n1, m2 = 2 * n2, m3 = 2 * n3;
+// ((ky*(n1+1) + kx)*U + blk)*n3 + p, k = zp_freq(n3/16, p).
+__global__ void k_full_store_pair(const zd* tmp, float4* dst, int n1, int n2, int n3, int U, int blk, int s3,
+                                  double scl) {
+  const int m3 = 2 * n3;
   const int nkx = n1 + 1, nky = n2 + 1;
-  const int64_t total = (int64_t)m1 * m2 * m3;
+  const int64_t total = (int64_t)nkx * nky * n3;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
-    const int kz = (int)(idx % m3);
-    const int64_t r = idx / m3;
-    const int kx = (int)(r % m1);
-    const int ky = (int)(r / m1);
-    const bool mx = kx > n1, my = ky > n2, mz = kz > n3;
-    const int kxo = mx ? m1 - kx : kx, kyo = my ? m2 - ky : ky, kzo = mz ? m3 - kz : kz;
-    const double sg = (double)((mx ? s1 : 1) * (my ? s2 : 1) * (mz ? s3 : 1)) * scl;
-    const zd v = tmp[kxo + (int64_t)nkx * (kyo + (int64_t)nky * kzo)];
-    float* d = dst + ((r * U + blk) * n3 + (kz >> 1)) * 4 + (kz & 1);
-    d[0] = (float)(v.x * sg);
-    d[2] = (float)(v.y * sg);
+    const int p = (int)(idx % n3);
+    const int k = zp_freq(n3 >> 4, p);
+    const int64_t r = idx / n3;
+    const int kx = (int)(r % nkx);
+    const int ky = (int)(r / nkx);
+    zd v[2];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+      const int kz = 2 * k + o;
+      const bool mz = kz > n3;
+      v[o] = scale(tmp[kx + (int64_t)nkx * (ky + (int64_t)nky * (mz ? m3 - kz : kz))], (double)(mz ? s3 : 1) * scl);
+    }
+    dst[(r * U + blk) * n3 + p] = make_float4((float)v[0].x, (float)v[1].x, (float)v[0].y, (float)v[1].y);
   }
 }
 
@@ -214,7 +216,7 @@ static marie_status check_parity_tucker(const marie_tucker_block& t, int n1, int
 
 // Build all blocks of one operator (N or K) into the handle's spectra.
 // Spectrum destinations of one operator: octant per precision (generic
-// path, K) and full block-interleaved (four-step path, N); null = not built.
+// path, K) and octant columns (four-step path, N); null = not built.
 struct SpecDst {
   cplx<double>* o64 = nullptr;
   cplx<float>* o32 = nullptr;
@@ -254,22 +256,22 @@ static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const d
   marie_status st = MARIE_OK;
   const int tabk = ncomp == 6 ? 0 : 2;   // N or K table (mirror signs)
   const BlockTab& bt = h->tab[tabk];
-  const int64_t full = (int64_t)8 * n1 * n2 * n3;
+  const int64_t full = (int64_t)nkx * nky * 2 * n3;
   auto store_block = [&](int id) {
     if (dst.o64) { k_oct_store<double><<<grid_for(oct), 256>>>(tmp, dst.o64 + id * oct, nkx, nky, nkz, scl); g_launches++; }
     if (dst.o32) { k_oct_store<float><<<grid_for(oct), 256>>>(tmp, dst.o32 + id * oct, nkx, nky, nkz, scl); g_launches++; }
-    const int s1 = bt.s1[id], s2 = bt.s2[id], s3 = bt.s3[id];
+    const int s3 = bt.s3[id];
     if (dst.f64) {
-      k_full_store<double><<<grid_for(full), 256>>>(tmp, dst.f64, n1, n2, n3, nblk, id, s1, s2, s3, scl);
+      k_full_store<double><<<grid_for(full), 256>>>(tmp, dst.f64, n1, n2, n3, nblk, id, s3, scl);
       g_launches++;
     }
     if (dst.f32) {
-      k_full_store_pair<<<grid_for(full), 256>>>(tmp, reinterpret_cast<float*>(dst.f32), n1, n2, n3, nblk, id, s1, s2,
-                                                  s3, scl);
+      k_full_store_pair<<<grid_for(full / 2), 256>>>(tmp, reinterpret_cast<float4*>(dst.f32), n1, n2, n3, nblk, id, s3,
+                                                     scl);
       g_launches++;
     }
     if (dst.fff) {
-      k_full_store<ff><<<grid_for(full), 256>>>(tmp, dst.fff, n1, n2, n3, nblk, id, s1, s2, s3, scl);
+      k_full_store<ff><<<grid_for(full), 256>>>(tmp, dst.fff, n1, n2, n3, nblk, id, s3, scl);
       g_launches++;
     }
   };
@@ -363,7 +365,7 @@ static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const d
 
 marie_status build_spectra(marie_vie* h, const marie_vie_desc* d) {
   const int64_t oct = (int64_t)(h->n1 + 1) * (h->n2 + 1) * (h->n3 + 1);
-  const int64_t full = (int64_t)8 * h->n1 * h->n2 * h->n3;
+  const int64_t full = (int64_t)(h->n1 + 1) * (h->n2 + 1) * 2 * h->n3;   // octant columns
   const bool fast = four_step_grid(h);
   if (h->precisions & 1) {
     MARIE_TRY(dev_alloc(h, (void**)&h->p64.GN, (size_t)h->nblkN * oct * sizeof(cplx<double>)));

@@ -8,15 +8,17 @@
 // start of every complex64 application of N or N^H, once for all the chunks
 // of right-hand sides of that application:
 //   P1[a, b, kz] = sum_c G[a, b, c] U3[c, kz]             (r1 r2 x 2n3)
-//   P2[a, ky, kz] = sum_b P1[a, b, kz] U2[b, ky]          (r1 x 2n2 x 2n3)
+//   P2[a, ky, kz] = sum_b P1[a, b, kz] U2[b, ky]          (r1 x (n2+1) x 2n3)
 //   G(ky, kx, kz) = sum_a P2[a, ky, kz] U1[a, kx] / (8 n1 n2 n3)
-// over the whole (2n)^3 grid (the factors are already circulant-extended and
-// transformed, assembly_fft_circ_tucker_pwl.m:50-58), written straight into
-// the pair layout: ((ky 2n1 + kx) U + blk) n3 + k holds (re G(2k), re
+// over the octant columns kx <= n1, ky <= n2 (the factors are already
+// circulant-extended and transformed, assembly_fft_circ_tucker_pwl.m:50-58),
+// written straight into the pair layout: ((ky (n1+1) + kx) U + blk) n3 + p, k =
+// zp_freq(n3/16, p), holds (re G(2k), re
 // G(2k+1), im G(2k), im G(2k+1)).  FP32 arithmetic, as the complex64 path.
 #include <algorithm>
 #include <vector>
 
+#include "fastpath.cuh"
 #include "internal.h"
 
 namespace marie {
@@ -51,7 +53,7 @@ __global__ void k_tkf2(const cplx<float>* __restrict__ P1, const cplx<float>* __
   }
 }
 
-// The last mode product is, for each ky, the product of U1^T (2n1 x r1)
+// The last mode product is, for each ky, the product of U1^T ((n1+1) x r1)
 // with the slab P2[:, ky, :] (r1 x 2n3).  A CTA takes one (ky, block) and a
 // tile of kTkX consecutive kx: its threads run over the frequency pairs k
 // (coalesced 16-byte stores), each holding the slab's two rank vectors for
@@ -70,7 +72,8 @@ __global__ void __launch_bounds__(128) k_tkf3(const cplx<float>* __restrict__ P2
     u[j * kTkMaxR + a] = U1[a + (int64_t)r1 * (kx0 + j)];
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < n3; k += blockDim.x) {
+  for (int p = threadIdx.x; p < n3; p += blockDim.x) {
+    const int k = zp_freq(n3 >> 4, p);
     cplx<float> p0[kTkMaxR], p1[kTkMaxR];
     const cplx<float>* q0 = P2 + (int64_t)r1 * (ky + (int64_t)m2 * (2 * k));
     const cplx<float>* q1 = q0 + (int64_t)r1 * m2;
@@ -92,7 +95,7 @@ __global__ void __launch_bounds__(128) k_tkf3(const cplx<float>* __restrict__ P2
         }
       }
       const int64_t col = (int64_t)ky * m1 + kx0 + j;
-      dst[(col * U + blk) * n3 + k] = make_float4(g0.x * scl, g1.x * scl, g0.y * scl, g1.y * scl);
+      dst[(col * U + blk) * n3 + p] = make_float4(g0.x * scl, g1.x * scl, g0.y * scl, g1.y * scl);
     }
   }
 }
@@ -144,7 +147,7 @@ marie_status tucker_keep_c64(marie_vie* h, const marie_tucker_block* tk) {
 
 marie_status tucker_expand_c64(marie_vie* h, cudaStream_t s) {
   TuckerDev& t = h->tkf;
-  const int m1 = 2 * h->n1, m2 = 2 * h->n2, m3 = 2 * h->n3, n3 = h->n3;
+  const int m1 = h->n1 + 1, m2 = h->n2 + 1, m3 = 2 * h->n3, n3 = h->n3;   // octant columns
   const int U = h->nblkN;
   const float scl = (float)(1.0 / (8.0 * (double)h->n1 * (double)h->n2 * (double)h->n3));
   float4* dst = reinterpret_cast<float4*>(h->p32.GNf);
