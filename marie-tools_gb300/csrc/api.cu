@@ -240,13 +240,13 @@ static marie_status choose_tiles(marie_vie* h, PrecState<T>& ps) {
   const int n3 = h->n3, C = h->C;
   const int sz = (int)sizeof(cplx<T>);
   int W = 16;
-  while (W > 1 && (size_t)n3 * (2 * C * W + 1) * sz > 100 * 1024) W /= 2;
+  while (W > 1 && (size_t)ps.m3 * (2 * C * W + 1) * sz > 100 * 1024) W /= 2;
   // MARIE_Z_TILE: z-pass tile width (power of two <= 16) if its shared
   // memory fits one CTA (227 KB)
   const int wz = env_int("MARIE_Z_TILE", 0);
   const size_t lim = kSmemOptin;
   if (wz >= 1 && wz <= 16 && (wz & (wz - 1)) == 0 && (size_t)n3 * (2 * C * wz + 2) * sz <= lim &&
-      kz4_smem<T>(n3, C, wz) <= lim)
+      kz4_smem<T>(ps.m3, C, wz) <= lim)
     W = wz;
   // The generic passes (any grid; K and K^H on every grid) with the
   // narrowest row tiles and a bundle of W right-hand sides must fit one CTA's
@@ -275,6 +275,8 @@ static marie_status choose_tiles(marie_vie* h, PrecState<T>& ps) {
   return MARIE_OK;
 }
 
+constexpr double kPadVolume = 3.0;    // see pad_c64
+
 struct CallTiles {
   int R, TY, TXY, TX, TZY;
 };
@@ -292,9 +294,10 @@ static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, 
   CallTiles t;
   const int Wz = ps.TX;
   t.R = pow2floor(std::max(1, std::min(Wz, nr)));
+  const int n1 = ps.m1, n2 = ps.m2;
   const int wxy = (sizeof(T) == 4 ? 16 : 8) * (fast ? 2 : 1);   // row-tile width of the x/y passes
-  t.TY = std::max(1, std::min(h->n2, wxy / t.R));
-  t.TXY = std::max(1, std::min(2 * h->n1, wxy / t.R));
+  t.TY = std::max(1, std::min(n2, wxy / t.R));
+  t.TXY = std::max(1, std::min(2 * n1, wxy / t.R));
   t.TZY = 1;
   if (fast && sizeof(T) == 4) {
     // slices of a column (xy4c.cuh): W = 32 elements per tile.  On short axes,
@@ -312,10 +315,10 @@ static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, 
       while (w > std::max(8, t.R) && ctas(w) < kSms) w /= 2;
       return w / t.R;
     };
-    t.TY = tile(h->n1, h->n2);
-    t.TZY = tile(h->n2, 2 * (int64_t)h->n1);
+    t.TY = tile(n1, h->n2);
+    t.TZY = tile(n2, 2 * (int64_t)n1);
   }
-  t.TX = std::max(1, std::min(2 * h->n1, Wz / t.R));
+  t.TX = std::max(1, std::min(2 * n1, Wz / t.R));
   // the complex64 PWL z pass shares each Green value among four elements
   if (fast && sizeof(T) == 4 && h->pwl) t.TX = std::max(t.TX, 4 / t.R);
   if (!fast) {   // generic passes: keep every tile within one CTA's shared memory
@@ -340,7 +343,8 @@ static void fill_axis(AxisTab<T>& dst, const AxisDev<T>& src) {
 
 template <typename T>
 static marie_status alloc_workspace(marie_vie* h, PrecState<T>& ps) {
-  const int64_t per = (int64_t)h->C * h->n3 * h->n2 * 2 * h->n1;  // T1 per rhs
+  const int64_t per = (int64_t)h->C * h->n3 * h->n2 * 2 * ps.m1;  // T1 per rhs
+  const int64_t perS = (int64_t)h->C * h->n3 * 2 * ps.m2 * 2 * ps.m1;
   int ws = std::max(1, std::min(h->max_rhs, env_int("MARIE_WS_RHS", 16)));
   const int Wz = ps.TX;
   if (ws > Wz) ws = (ws + Wz - 1) / Wz * Wz;   // whole bundles
@@ -348,7 +352,7 @@ static marie_status alloc_workspace(marie_vie* h, PrecState<T>& ps) {
   const int64_t alloc = (int64_t)(ws + Wz - 1) / Wz * Wz;   // any chunk of <= ws rhs fits whole bundles
   ps.ws_cap = (int)alloc;
   MARIE_TRY(dev_alloc(h, (void**)&ps.T1, (size_t)alloc * per * sizeof(cplx<T>)));
-  MARIE_TRY(dev_alloc(h, (void**)&ps.S, (size_t)alloc * per * 2 * sizeof(cplx<T>)));
+  MARIE_TRY(dev_alloc(h, (void**)&ps.S, (size_t)alloc * perS * sizeof(cplx<T>)));
   return MARIE_OK;
 }
 
@@ -424,9 +428,9 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
   smem_opt_in_device((const void*)k_inv_x<double>, done[7]);
   MvArgs<T> a;
   memset(&a, 0, sizeof(a));
-  a.n1 = h->n1;
-  a.n2 = h->n2;
-  a.n3 = h->n3;
+  a.n1 = ps.m1;
+  a.n2 = ps.m2;
+  a.n3 = ps.m3;
   a.g1 = h->n1;
   a.g2 = h->n2;
   a.g3 = h->n3;
@@ -440,7 +444,7 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
   if (mode != MV_GRID && !env_int("MARIE_NO_PRUNE", 0)) {
     a.row_live = h->row_live;
     a.z_live = h->z_live;
-    a.rowq = h->rowq;
+    a.rowq = ps.padded ? ps.rowq : h->rowq;
     a.zq = h->zq;
   }
   a.chi = ps.chi;
@@ -460,8 +464,8 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
   }
   for (int r0 = 0; r0 < nrhs; r0 += ps.ws_rhs) {
     const int nr = std::min(ps.ws_rhs, nrhs - r0);
-    const bool fast = four_step_edge(n1) && four_step_edge(n2) && four_step_edge(n3) &&
-                      (op == OP_N || op == OP_N_ADJ) && !env_int("MARIE_GENERIC_FFT", 0);
+    // a padded state has the four-step passes only
+    const bool fast = four_step_op(h, ps, op) && (ps.padded || !env_int("MARIE_GENERIC_FFT", 0));
     const CallTiles ct = call_tiles(h, ps, nr, fast);
     const int nb = (nr + ct.R - 1) / ct.R;
     a.R = ct.R;
@@ -477,7 +481,7 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
     a.active = active ? active + r0 : nullptr;
     a.addend = addend ? addend + (int64_t)r0 * out_rs : nullptr;
     if (fast) {
-      a.G = ps.GNf;
+      a.G = isK ? ps.GKf : ps.GNf;
       MARIE_TRY(launch_fast_chunk<T>(h, op, a, nb, stream, (ev && r0 == 0) ? ev : nullptr));
       continue;
     }
@@ -626,6 +630,49 @@ static marie_status validate_desc(const marie_vie_desc* d, std::vector<int64_t>&
   return MARIE_OK;
 }
 
+// complex64 on a grid that is not 16*NB: run the four-step passes on the next
+// multiples of 16 (the operator is a convolution, so any circulant of size 2m >=
+// 2n - 1 with zeros at the offsets n..m-1 gives the same on the grid, embed.h;
+// rows, slices and columns beyond the grid are never stored or read).  The
+// generic passes take four to five times as long per grid point (60 x 77 x 90
+// PWL, three right-hand sides: 6.5 ms against 1.9; 24^3 PWL one: 91 against 81
+// us at 2.4 times the volume; 17 x 40 x 40 PWL four: 491 against 339 at 2.7), so
+// padding pays up to about three times the volume.  Not under a memory cap, nor
+// where the larger work arrays and spectra would not fit easily: the generic
+// passes need less.  MARIE_GENERIC_FFT=1 at create keeps the generic passes.
+static marie_status pad_c64(marie_vie* h, const std::vector<int64_t>& idxS) {
+  PrecState<float>& ps = h->p32;
+  if (four_step_grid(h) || h->mem_cap > 0 || env_int("MARIE_GENERIC_FFT", 0)) return MARIE_OK;
+  const int n[3] = {h->n1, h->n2, h->n3};
+  int m[3];
+  double vol = 1;
+  for (int d = 0; d < 3; ++d) {
+    if (n[d] > 128) return MARIE_OK;
+    m[d] = (n[d] + 15) / 16 * 16;
+    vol *= (double)m[d] / n[d];
+  }
+  if (vol > kPadVolume) return MARIE_OK;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return MARIE_OK; }
+  const double rhs = std::max(1, std::min(h->max_rhs, env_int("MARIE_WS_RHS", 16))) + 16.0;
+  const double need = 8.0 * ((h->nblkN + (h->has_K ? h->nblkK : 0)) * (m[0] + 1.0) * (m[1] + 1.0) * 2.0 * m[2] +
+                             rhs * h->C * n[2] * (2.0 * m[0]) * (n[1] + 2.0 * m[1]));
+  if (need > 0.25 * (double)free_b) return MARIE_OK;
+  ps.m1 = m[0];
+  ps.m2 = m[1];
+  ps.m3 = m[2];
+  ps.padded = true;
+  const int nb = m[1] / 16;
+  std::vector<uint16_t> rq((size_t)h->n3 * 8, 0);
+  for (int64_t v : idxS) {
+    const int y = (int)((v / h->n1) % h->n2), z = (int)(v / ((int64_t)h->n1 * h->n2));
+    rq[(size_t)z * 8 + y % nb] |= (uint16_t)(1u << (y / nb));
+  }
+  MARIE_TRY(dev_alloc(h, (void**)&ps.rowq, rq.size() * sizeof(uint16_t)));
+  MARIE_CUDA_TRY(cudaMemcpy(ps.rowq, rq.data(), rq.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
+  return MARIE_OK;
+}
+
 // Handle for a grid the FFT passes take as given (marie_vie_create decides
 // whether the caller's grid is first embedded in a larger one, embed.h).
 static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
@@ -727,6 +774,13 @@ static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
   if ((st = dev_alloc(h, (void**)&h->wpow, h->Ns * sizeof(double))) != MARIE_OK) return fail(st);
   cudaMemcpy(h->wpow, wpow.data(), h->Ns * sizeof(double), cudaMemcpyHostToDevice);
   (void)e0;
+  auto own_dims = [&](auto& ps) { ps.m1 = h->n1; ps.m2 = h->n2; ps.m3 = h->n3; };
+  own_dims(h->p64);
+  own_dims(h->pff);
+  own_dims(h->p32);
+  if (d->precisions & 2) {
+    if ((st = pad_c64(h, idxS)) != MARIE_OK) return fail(st);
+  }
   for (int pr = 0; pr < 3; ++pr) {
     if (!(d->precisions & (1 << pr))) continue;
     if (pr == 2) {
@@ -751,9 +805,9 @@ static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
       if ((st = alloc_workspace(h, ps)) != MARIE_OK) return fail(st);
     } else {
       PrecState<float>& ps = h->p32;
-      if ((st = build_axis(h, h->n1, ps.ax)) != MARIE_OK) return fail(st);
-      if ((st = build_axis(h, h->n2, ps.ay)) != MARIE_OK) return fail(st);
-      if ((st = build_axis(h, h->n3, ps.az)) != MARIE_OK) return fail(st);
+      if ((st = build_axis(h, ps.m1, ps.ax)) != MARIE_OK) return fail(st);
+      if ((st = build_axis(h, ps.m2, ps.ay)) != MARIE_OK) return fail(st);
+      if ((st = build_axis(h, ps.m3, ps.az)) != MARIE_OK) return fail(st);
       std::vector<cplx<float>> chif(h->Ns);
       for (int64_t s = 0; s < h->Ns; ++s) chif[s] = cplx<float>{(float)chi[s].x, (float)chi[s].y};
       if ((st = dev_alloc(h, (void**)&ps.chi, h->Ns * sizeof(cplx<float>))) != MARIE_OK) return fail(st);
@@ -789,7 +843,7 @@ static marie_status autotune_state(marie_vie* h, PrecState<T>& ps, const void* x
                                    cudaStream_t s, int32_t* widths, double* ms, int32_t cap, int32_t* count) {
   const int C = h->C;
   const size_t sz = sizeof(cplx<T>);
-  const bool fast = four_step_grid(h) && !env_int("MARIE_GENERIC_FFT", 0);
+  const bool fast = ps.padded || (four_step_grid(h) && !env_int("MARIE_GENERIC_FFT", 0));
   const int keep = ps.TX;
   cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
@@ -800,7 +854,7 @@ static marie_status autotune_state(marie_vie* h, PrecState<T>& ps, const void* x
   for (int W = 1; W <= 16 && st == MARIE_OK; W *= 2) {
     if ((ps.ws_rhs + W - 1) / W * W > ps.ws_cap) continue;
     if (fast) {
-      if (kz4_smem<T>(h->n3, C, W) > kSmemOptin) continue;
+      if (kz4_smem<T>(ps.m3, C, W) > kSmemOptin) continue;
     } else {
       const GenericSmem g = generic_smem(h->n1, h->n2, h->n3, C, sz, 1, 1, 1, W);
       if (g.x > kSmemOptin || g.y > kSmemOptin || g.z > kSmemOptin) continue;

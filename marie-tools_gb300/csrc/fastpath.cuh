@@ -102,7 +102,7 @@ void launch_z_nb(int nb, int op, const MvArgs<T>& a, dim3 g, size_t smem, cudaSt
 // launch_matvec_ev.  Tiles in `a` are set by the caller.
 template <typename T>
 marie_status launch_fast_chunk(marie_vie* h, int op, MvArgs<T>& a, int nb, cudaStream_t stream, cudaEvent_t* ev) {
-  const int n1 = h->n1, n2 = h->n2, n3 = h->n3, C = h->C;
+  const int n1 = a.n1, n2 = a.n2, n3 = a.n3, C = h->C;
   const size_t sz = sizeof(cplx<T>);
   constexpr bool c64 = std::is_same<T, float>::value;
   const size_t smx = (size_t)(n1 + (size_t)2 * a.TY * a.R * (n1 + 1)) * sz;

@@ -84,11 +84,15 @@ void launch_y_nb(int nb, bool inv, const MvArgs<T>& a, dim3 g, size_t smem, cuda
 #undef Y_CALL
 }
 
-// The four-step path serves N (op 0) and N^H (op 1).
+// The four-step path serves N (op 0) and N^H (op 1), in complex64 also K and K^H.
 template <typename T, bool PWL, int NB>
 void launch_z_one(int op, const MvArgs<T>& a, dim3 g, size_t smem, cudaStream_t s) {
   if (op == OP_N) launch_z4<T, NB, PWL, 0>(a, g, smem, s);
-  else launch_z4<T, NB, PWL, 1>(a, g, smem, s);
+  else if (op == OP_N_ADJ) launch_z4<T, NB, PWL, 1>(a, g, smem, s);
+  if constexpr (std::is_same<T, float>::value) {
+    if (op == OP_K) launch_z4<T, NB, PWL, 2>(a, g, smem, s);
+    else if (op == OP_K_ADJ) launch_z4<T, NB, PWL, 3>(a, g, smem, s);
+  }
 }
 
 }  // namespace marie

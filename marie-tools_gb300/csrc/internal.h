@@ -60,11 +60,15 @@ struct PrecState {
   cplx<T>* GN = nullptr;      // nblkN * oct
   cplx<T>* GK = nullptr;      // nblkK * oct
   cplx<T>* GNf = nullptr;     // octant columns [ky <= n2][kx <= n1], each [kz][blk] (four-step grids; complex64: pair layout)
+  cplx<T>* GKf = nullptr;     // the same for K (complex64)
   cplx<T>* T1 = nullptr;      // ws_rhs * C * n3 * n2 * 2n1
   cplx<T>* S = nullptr;       // ws_rhs * C * 2n2 * n3 * 2n1
   int ws_rhs = 0;             // right-hand sides per matvec chunk
   int ws_cap = 0;             // right-hand sides the work arrays hold (whole z-tile bundles)
   int TY = 1, TXY = 1, TX = 1;
+  int m1 = 0, m2 = 0, m3 = 0; // transform lengths: the grid's edges, or multiples of 16 above them (padded)
+  bool padded = false;        // complex64 on a grid that is not 16*NB: four-step passes on m1 x m2 x m3
+  uint16_t* rowq = nullptr;   // row_live in the four-step order of m2 (padded)
 };
 
 // Tucker factors kept on the device (FP32) for the per-application
@@ -227,6 +231,12 @@ inline int generic_tile_cap(int n, int mult, int R, size_t sz) {
 inline bool four_step_edge(int n) { return n % 16 == 0 && n / 16 >= 1 && n / 16 <= 8; }
 inline bool four_step_grid(const marie_vie* h) {
   return four_step_edge(h->n1) && four_step_edge(h->n2) && four_step_edge(h->n3);
+}
+// The four-step passes run operator op in precision T: N and N^H on every
+// four-step grid, K and K^H and padded grids in complex64.
+template <typename T>
+inline bool four_step_op(const marie_vie* h, const PrecState<T>& ps, int op) {
+  return (four_step_grid(h) || ps.padded) && (op == OP_N || op == OP_N_ADJ || sizeof(T) == 4);
 }
 
 }  // namespace marie

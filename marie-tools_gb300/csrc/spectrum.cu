@@ -19,27 +19,50 @@ namespace marie {
 typedef cplx<double> zd;
 
 // out[o][k][i] = sum_j in[o][j][i] * e(j,k),  e(0,k) = 1,
-// e(j,k) = w_2n^{jk} + s * w_2n^{-jk}  (j >= 1), k in [0, n]
-__global__ void k_circ_axis(const zd* __restrict__ in, zd* __restrict__ out, int n, int s, int64_t inner,
-                            int64_t outer, const zd* __restrict__ w2n) {
-  const int64_t total = outer * (n + 1) * inner;
+// e(j,k) = w_2m^{jk} + s * w_2m^{-jk}  (1 <= j < n), k in [0, m], m >= n: the
+// circulant extension of length 2m, zero at the offsets n..m-1
+__global__ void k_circ_axis(const zd* __restrict__ in, zd* __restrict__ out, int n, int m, int s, int64_t inner,
+                            int64_t outer, const zd* __restrict__ w2m) {
+  const int64_t total = outer * (m + 1) * inner;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t ii = idx % inner;
     const int64_t r = idx / inner;
-    const int k = (int)(r % (n + 1));
-    const int64_t o = r / (n + 1);
+    const int k = (int)(r % (m + 1));
+    const int64_t o = r / (m + 1);
     const zd* src = in + o * n * inner + ii;
     zd acc = src[0];
     for (int j = 1; j < n; ++j) {
-      const int e = (int)(((int64_t)j * k) % (2 * n));
-      const zd w = w2n[e];
+      const int e = (int)(((int64_t)j * k) % (2 * m));
+      const zd w = w2m[e];
       const zd v = src[(int64_t)j * inner];
       // v * (w + s*conj(w))
       const zd ws = {w.x + s * w.x, w.y - s * w.y};
       acc = acc + v * ws;
     }
     out[idx] = acc;
+  }
+}
+
+// The inverse of k_circ_axis with m = n: out[o][j][i], j < n, from the values
+// in[o][k][i] at the octant frequencies k in [0, n].
+__global__ void k_circ_inv(const zd* __restrict__ in, zd* __restrict__ out, int n, int s, int64_t inner,
+                           int64_t outer, const zd* __restrict__ w2n) {
+  const int64_t total = outer * n * inner;
+  const double h = 0.5 / n;
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t ii = idx % inner;
+    const int64_t r = idx / inner;
+    const int j = (int)(r % n);
+    const int64_t o = r / n;
+    const zd* src = in + o * (n + 1) * inner + ii;
+    zd acc = (j & 1) ? src[0] - src[(int64_t)n * inner] : src[0] + src[(int64_t)n * inner];
+    for (int k = 1; k < n; ++k) {
+      const zd w = w2n[(int)(((int64_t)j * k) % (2 * n))];
+      acc = acc + src[(int64_t)k * inner] * zd{w.x + s * w.x, -(w.y - s * w.y)};   // conj(w) + s w
+    }
+    out[idx] = scale(acc, h);
   }
 }
 
@@ -223,6 +246,7 @@ struct SpecDst {
   cplx<double>* f64 = nullptr;
   cplx<float>* f32 = nullptr;
   cplx<ff>* fff = nullptr;
+  cplx<float>* pad = nullptr;    // complex64 octant columns of the padded lengths m (PrecState::padded)
 };
 
 static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const double* dense, int ncomp,
@@ -257,6 +281,53 @@ static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const d
   const int tabk = ncomp == 6 ? 0 : 2;   // N or K table (mirror signs)
   const BlockTab& bt = h->tab[tabk];
   const int64_t full = (int64_t)nkx * nky * 2 * n3;
+  // padded complex64 spectrum: transform lengths m, tables, scratch (pa: the
+  // block at offsets; pb, pc: after one and two axes; pt: its octant)
+  const int m[3] = {h->p32.m1, h->p32.m2, h->p32.m3}, nn[3] = {n1, n2, n3};
+  const int64_t poct = (int64_t)(m[0] + 1) * (m[1] + 1) * (m[2] + 1);
+  const double pscl = 1.0 / (8.0 * (double)m[0] * (double)m[1] * (double)m[2]);
+  zd *pa = nullptr, *pb = nullptr, *pc = nullptr, *pt = nullptr, *wn[3] = {}, *wm[3] = {};
+  auto root_table = [&](zd** p, int n) -> marie_status {
+    MARIE_TRY(salloc(p, 2 * n));
+    std::vector<zd> w(2 * n);
+    for (int k = 0; k < 2 * n; ++k) {
+      const long double ang = -3.141592653589793238462643383279502884L * (long double)k / (long double)n;
+      w[k] = zd{(double)std::cos(ang), (double)std::sin(ang)};
+    }
+    cudaMemcpy(*p, w.data(), 2 * n * sizeof(zd), cudaMemcpyHostToDevice);
+    return MARIE_OK;
+  };
+  auto pad_alloc = [&]() -> marie_status {
+    if (!dst.pad) return MARIE_OK;
+    for (int d = 0; d < 3; ++d) {
+      MARIE_TRY(root_table(&wn[d], nn[d]));
+      MARIE_TRY(root_table(&wm[d], m[d]));
+    }
+    MARIE_TRY(salloc(&pa, nD));
+    MARIE_TRY(salloc(&pb, (int64_t)(m[0] + 1) * (n2 + 1) * (n3 + 1)));
+    MARIE_TRY(salloc(&pc, (int64_t)(m[0] + 1) * (m[1] + 1) * (n3 + 1)));
+    MARIE_TRY(salloc(&pt, poct));
+    return MARIE_OK;
+  };
+  // block: its values at the offsets (dense), or null: recovered from tmp
+  auto store_pad = [&](int id, const zd* block) {
+    if (!dst.pad) return;
+    const int s1 = bt.s1[id], s2 = bt.s2[id], s3 = bt.s3[id];
+    if (!block) {
+      k_circ_inv<<<grid_for((int64_t)nkx * nky * n3), 256>>>(tmp, pc, n3, s3, (int64_t)nkx * nky, 1, wn[2]);
+      k_circ_inv<<<grid_for((int64_t)nkx * n2 * n3), 256>>>(pc, pb, n2, s2, nkx, n3, wn[1]);
+      k_circ_inv<<<grid_for(nD), 256>>>(pb, pa, n1, s1, 1, (int64_t)n2 * n3, wn[0]);
+      g_launches += 3;
+      block = pa;
+    }
+    const int64_t kx = m[0] + 1, ky = m[1] + 1;
+    k_circ_axis<<<grid_for(kx * n2 * n3), 256>>>(block, pb, n1, m[0], s1, 1, (int64_t)n2 * n3, wm[0]);
+    k_circ_axis<<<grid_for(kx * ky * n3), 256>>>(pb, pc, n2, m[1], s2, kx, n3, wm[1]);
+    k_circ_axis<<<grid_for(poct), 256>>>(pc, pt, n3, m[2], s3, kx * ky, 1, wm[2]);
+    k_full_store_pair<<<grid_for(kx * ky * m[2]), 256>>>(pt, reinterpret_cast<float4*>(dst.pad), m[0], m[1], m[2], nblk,
+                                                         id, s3, pscl);
+    g_launches += 4;
+  };
   auto store_block = [&](int id) {
     if (dst.o64) { k_oct_store<double><<<grid_for(oct), 256>>>(tmp, dst.o64 + id * oct, nkx, nky, nkz, scl); g_launches++; }
     if (dst.o32) { k_oct_store<float><<<grid_for(oct), 256>>>(tmp, dst.o32 + id * oct, nkx, nky, nkz, scl); g_launches++; }
@@ -277,23 +348,15 @@ static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const d
   };
   do {
     if ((st = salloc(&tmp, oct)) != MARIE_OK) break;
+    if ((st = pad_alloc()) != MARIE_OK) break;
+    // a padded handle without complex128 needs nothing on the grid's own lengths
+    const bool own = dst.o64 || dst.o32 || dst.f64 || dst.f32 || dst.fff;
     if (dense) {
       if ((st = salloc(&a, nD)) != MARIE_OK) break;
       if ((st = salloc(&b, (int64_t)nkx * nky * n3)) != MARIE_OK) break;
-      // w_2n tables per axis
-      zd* ws[3] = {nullptr, nullptr, nullptr};
-      const int ns[3] = {n1, n2, n3};
-      for (int d = 0; d < 3 && st == MARIE_OK; ++d) {
-        if ((st = salloc(&ws[d], 2 * ns[d])) != MARIE_OK) break;
-        std::vector<zd> w(2 * ns[d]);
-        for (int k = 0; k < 2 * ns[d]; ++k) {
-          const long double ang = -3.141592653589793238462643383279502884L * (long double)k / (long double)ns[d];
-          w[k] = zd{(double)std::cos(ang), (double)std::sin(ang)};
-        }
-        cudaMemcpy(ws[d], w.data(), 2 * ns[d] * sizeof(zd), cudaMemcpyHostToDevice);
-      }
-      if (st != MARIE_OK) break;
-      w1 = ws[0]; w2 = ws[1]; w3 = ws[2];
+      if ((st = root_table(&w1, n1)) != MARIE_OK || (st = root_table(&w2, n2)) != MARIE_OK ||
+          (st = root_table(&w3, n3)) != MARIE_OK)
+        break;
       zd* c = nullptr;
       if ((st = salloc(&c, (int64_t)nkx * nky * n3)) != MARIE_OK) break;
       for (int id = 0; id < nblk; ++id) {
@@ -307,13 +370,14 @@ static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const d
           st = MARIE_ERR_CUDA;
           break;
         }
-        k_circ_axis<<<grid_for((int64_t)nkx * n2 * n3), 256>>>(a, b, n1, bt.s1[id], 1, (int64_t)n2 * n3, w1);
-        g_launches++;
-        k_circ_axis<<<grid_for((int64_t)nkx * nky * n3), 256>>>(b, c, n2, bt.s2[id], nkx, n3, w2);
-        g_launches++;
-        k_circ_axis<<<grid_for(oct), 256>>>(c, tmp, n3, bt.s3[id], (int64_t)nkx * nky, 1, w3);
-        g_launches++;
-        store_block(id);
+        if (own) {
+          k_circ_axis<<<grid_for((int64_t)nkx * n2 * n3), 256>>>(a, b, n1, n1, bt.s1[id], 1, (int64_t)n2 * n3, w1);
+          k_circ_axis<<<grid_for((int64_t)nkx * nky * n3), 256>>>(b, c, n2, n2, bt.s2[id], nkx, n3, w2);
+          k_circ_axis<<<grid_for(oct), 256>>>(c, tmp, n3, n3, bt.s3[id], (int64_t)nkx * nky, 1, w3);
+          g_launches += 3;
+          store_block(id);
+        }
+        store_pad(id, a);
         if (cudaGetLastError() != cudaSuccess) { set_error("spectrum kernel launch failed"); st = MARIE_ERR_CUDA; break; }
         cudaDeviceSynchronize();
       }
@@ -354,6 +418,7 @@ static marie_status build_op(marie_vie* h, const marie_tucker_block* tk, const d
         k_tk3<<<grid_for(oct), 256>>>(b, dU1, tmp, t.r1, nkx, nky, nkz);
         g_launches++;
         store_block(id);
+        store_pad(id, nullptr);
         if (cudaGetLastError() != cudaSuccess) { set_error("spectrum kernel launch failed"); st = MARIE_ERR_CUDA; break; }
         cudaDeviceSynchronize();
       }
@@ -373,9 +438,16 @@ marie_status build_spectra(marie_vie* h, const marie_vie_desc* d) {
     if (fast) MARIE_TRY(dev_alloc(h, (void**)&h->p64.GNf, (size_t)h->nblkN * full * sizeof(cplx<double>)));
   }
   if (h->precisions & 2) {
-    MARIE_TRY(dev_alloc(h, (void**)&h->p32.GN, (size_t)h->nblkN * oct * sizeof(cplx<float>)));
-    if (h->has_K) MARIE_TRY(dev_alloc(h, (void**)&h->p32.GK, (size_t)h->nblkK * oct * sizeof(cplx<float>)));
-    if (fast) MARIE_TRY(dev_alloc(h, (void**)&h->p32.GNf, (size_t)h->nblkN * full * sizeof(cplx<float>)));
+    const PrecState<float>& ps = h->p32;
+    const int64_t cols = (int64_t)(ps.m1 + 1) * (ps.m2 + 1) * 2 * ps.m3;
+    if (!ps.padded) {
+      MARIE_TRY(dev_alloc(h, (void**)&h->p32.GN, (size_t)h->nblkN * oct * sizeof(cplx<float>)));
+      if (h->has_K) MARIE_TRY(dev_alloc(h, (void**)&h->p32.GK, (size_t)h->nblkK * oct * sizeof(cplx<float>)));
+    }
+    if (fast || ps.padded) {
+      MARIE_TRY(dev_alloc(h, (void**)&h->p32.GNf, (size_t)h->nblkN * cols * sizeof(cplx<float>)));
+      if (h->has_K) MARIE_TRY(dev_alloc(h, (void**)&h->p32.GKf, (size_t)h->nblkK * cols * sizeof(cplx<float>)));
+    }
   }
   if (h->precisions & 4)   // float-float: four-step path only (N and N^H)
     MARIE_TRY(dev_alloc(h, (void**)&h->pff.GNf, (size_t)h->nblkN * full * sizeof(cplx<ff>)));
@@ -383,13 +455,14 @@ marie_status build_spectra(marie_vie* h, const marie_vie_desc* d) {
   dN.o64 = h->p64.GN;
   dN.o32 = h->p32.GN;
   dN.f64 = h->p64.GNf;
-  dN.f32 = h->p32.GNf;
+  (h->p32.padded ? dN.pad : dN.f32) = h->p32.GNf;
   dN.fff = h->pff.GNf;
   MARIE_TRY(build_op(h, d->tucker_N, d->tucker_N ? nullptr : d->dense_N, 6, dN));
   if (h->has_K) {
     SpecDst dK;
     dK.o64 = h->p64.GK;
     dK.o32 = h->p32.GK;
+    (h->p32.padded ? dK.pad : dK.f32) = h->p32.GKf;
     MARIE_TRY(build_op(h, d->tucker_K, d->tucker_K ? nullptr : d->dense_K, 3, dK));
   }
   return MARIE_OK;
