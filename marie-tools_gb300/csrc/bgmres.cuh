@@ -22,7 +22,8 @@
 //
 // The projections, updates, Gram matrices and combinations are GEMMs of a
 // tall (N_b rows) operand with (j+1)p or p columns: cuBLAS complex GEMMs on
-// the tensor cores (FP32 emulated by BF16x9 products, FP32 accumulation;
+// the tensor cores (FP32 emulated by BF16x9 products, FP32 accumulation; up to
+// sixteen right-hand sides the kernels of bsmall.cuh instead;
 // MARIE_BLOCK_GEMM=fp32 runs them on the FP32 pipe instead;
 // MARIE_BLOCK_PROJ=tcgen05 runs the projections on bproj.cu's kernel).  The small
 // p x p and (j+2)p x p matrices move through pinned, device-mapped host
@@ -33,6 +34,7 @@
 #include <cublas_v2.h>
 
 #include "blocklsq.h"
+#include "bsmall.cuh"
 
 namespace marie {
 
@@ -256,6 +258,7 @@ struct BlockWork {
   int64_t part_cap = 0;
   float* tpart = nullptr;      // partial sums of the tensor-core path
   int64_t tpart_floats = 0;
+  bool tall = false;           // few right-hand sides: the kernels of bsmall.cuh
   bool tc = false;             // projections on the tensor-core kernel (MARIE_BLOCK_PROJ=tcgen05)
 };
 
@@ -283,7 +286,16 @@ static bool proj_tcgen05() {
 
 // H (m x p, ld m) = A^H B for the N_b-row blocks A (m columns) and B (p columns)
 static marie_status proj_cn(marie_vie* h, BlockWork& w, cublasHandle_t bl, int64_t m, const cplx<float>* A,
-                            const cplx<float>* B, cplx<float>* H, cudaStream_t s) {
+                            const cplx<float>* B, cplx<float>* H, cudaStream_t s, bool check = false) {
+  if (w.tall) {
+    int* flag = nullptr;
+    if (check) {
+      unsigned char* qd = nullptr;
+      MARIE_CUDA_TRY(cudaHostGetDevicePointer((void**)&qd, h->bio, 0));
+      flag = (int*)(qd + bio_err(w.p, w.mb));
+    }
+    return tall_cn(w.Nb, (int)m, w.p, A, B, H, w.part, flag, s);
+  }
   if (w.tc) {
     unsigned char* qd = nullptr;
     MARIE_CUDA_TRY(cudaHostGetDevicePointer((void**)&qd, h->bio, 0));
@@ -291,6 +303,14 @@ static marie_status proj_cn(marie_vie* h, BlockWork& w, cublasHandle_t bl, int64
                          (int*)(qd + bio_err(w.p, w.mb)), s);
   }
   return cgemm_cn(bl, m, w.p, w.Nb, A, w.Nb, B, w.Nb, H, m, w.part, w.part_cap, s);
+}
+
+// C (N_b x p) = alpha A X + beta C, A N_b x m, X m x p; alpha +-1, beta 0 or 1
+static marie_status comb(BlockWork& w, cublasHandle_t bl, int64_t m, float alpha, const cplx<float>* A,
+                         const cplx<float>* X, float beta, cplx<float>* C, cudaStream_t s) {
+  if (w.tall) return tall_comb(w.Nb, (int)m, w.p, alpha, A, X, beta, C, s);
+  return cgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, w.Nb, w.p, m, cuComplex{alpha, 0.f}, A, w.Nb, X, m, cuComplex{beta, 0.f},
+               C, w.Nb);
 }
 
 // after a synchronisation: the status word (1: a tensor-core wait expired,
@@ -321,7 +341,6 @@ static marie_status block_qr(marie_vie* h, BlockWork& w, cublasHandle_t bl, cplx
                              std::vector<zc>& R, cudaStream_t s) {
   const int p = w.p;
   const int64_t Nb = w.Nb;
-  const cuComplex one = {1.f, 0.f}, zero = {0.f, 0.f};
   const unsigned char* hb = h->bio;
   R.assign((size_t)p * p, zc(0, 0));
   for (int i = 0; i < p; ++i) R[i + (size_t)p * i] = 1.0;
@@ -332,7 +351,8 @@ static marie_status block_qr(marie_vie* h, BlockWork& w, cublasHandle_t bl, cplx
     // the Gram matrix in cuBLAS's FP32-accurate products: the Cholesky
     // factor needs its small eigenvalues (the tensor-core kernel's ~1e-6
     // relative error is enough for the projections, not here)
-    MARIE_TRY(cgemm_cn(bl, p, p, Nb, a, Nb, a, Nb, w.Gm, p, w.part, w.part_cap, s));
+    if (w.tall) MARIE_TRY(tall_cn(Nb, p, p, a, a, w.Gm, w.part, nullptr, s));
+    else MARIE_TRY(cgemm_cn(bl, p, p, Nb, a, Nb, a, Nb, w.Gm, p, w.part, w.part_cap, s));
     MARIE_TRY(bio_move(h, bio_gm(p, w.mb), w.Gm, (size_t)p * p * 8, true, s));
     MARIE_CUDA_TRY(cudaStreamSynchronize(s));
     MARIE_TRY(tc_check(h, w));
@@ -373,7 +393,7 @@ static marie_status block_qr(marie_vie* h, BlockWork& w, cublasHandle_t bl, cplx
     cplx<float>* up = reinterpret_cast<cplx<float>*>(h->bio + bio_up(p, w.mb));
     to_c64(Ri, up);
     MARIE_TRY(bio_move(h, bio_up(p, w.mb), w.Sm, (size_t)p * p * 8, false, s));
-    MARIE_TRY(cgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, Nb, p, p, one, a, Nb, w.Sm, p, zero, b, Nb));
+    MARIE_TRY(comb(w, bl, p, 1.f, a, w.Sm, 0.f, b, s));
     R = tri_mul(Rk, R, p);
     std::swap(a, b);
     // the pinned upload area is rewritten by the next pass only after the
@@ -398,7 +418,9 @@ static marie_status block_work_alloc(marie_vie* h, BlockWork& w, int pmax, int m
   MARIE_TRY(sc.get(&w.Gm, (size_t)pmax * pmax));
   MARIE_TRY(sc.get(&w.Sm, (size_t)(mb + 1) * pmax * pmax));
   MARIE_TRY(sc.get(&w.map, (size_t)pmax + 1));
-  w.part_cap = (int64_t)65 * mb * pmax * pmax;
+  // a refinement step may solve fewer columns than pmax and take bsmall.cuh then
+  const int64_t ps = std::min(pmax, kTallMax);
+  w.part_cap = std::max((int64_t)65 * mb * pmax * pmax, (int64_t)kTallCtas * mb * ps * ps);
   MARIE_TRY(sc.get(&w.part, (size_t)w.part_cap));
   w.tpart_floats = block_gemm_part_floats(Nb, mb * std::min(pmax, 64));
   if (pmax <= 64 && Nb % 2 == 0 && proj_tcgen05()) MARIE_TRY(sc.get(&w.tpart, (size_t)w.tpart_floats));
@@ -419,9 +441,9 @@ static marie_status bgmres_core(marie_vie* h, const std::vector<int>& cols, cons
   w.p = p;
   w.tc = p <= 64 && Nb % 2 == 0 && w.tpart != nullptr;
   MARIE_TRY(bio_reserve(h, bio_need(p, mb)));
+  w.tall = !w.tc && tall_fits((int64_t)(mb + 1) * p, p) && blas_mode() == std::string("bf16x9");
   cublasHandle_t bl = nullptr;
-  MARIE_TRY(blas_handle(h, s, &bl));
-  const cuComplex one = {1.f, 0.f}, zero = {0.f, 0.f}, mone = {-1.f, 0.f};
+  if (!w.tall) MARIE_TRY(blas_handle(h, s, &bl));
   // rhs map and the residual block in complex64
   MARIE_CUDA_TRY(cudaStreamSynchronize(s));
   *reinterpret_cast<volatile int*>(h->bio + bio_err(p, mb)) = 0;
@@ -446,7 +468,7 @@ static marie_status bgmres_core(marie_vie* h, const std::vector<int>& cols, cons
       MARIE_TRY(launch_matvec<float>(h, sc.adjoint ? MV_VIE_ADJ : MV_VIE, sc.adjoint ? OP_N_ADJ : OP_N, Vj, Nb, w.W,
                                      Nb, p, nullptr, s));
       ++*matvecs;
-      {
+      if (!w.tall) {   // the projection kernel of bsmall.cuh checks W itself
         unsigned char* qd = nullptr;
         MARIE_CUDA_TRY(cudaHostGetDevicePointer((void**)&qd, h->bio, 0));
         k_check_finite<<<vgrid(2 * (int64_t)p * Nb, 1).x, 256, 0, s>>>(reinterpret_cast<const float*>(w.W),
@@ -456,16 +478,15 @@ static marie_status bgmres_core(marie_vie* h, const std::vector<int>& cols, cons
       }
       if (prof.on) cudaEventRecord(prof.ev[1], s);
       const int64_t M = (int64_t)(j + 1) * p;
-      MARIE_TRY(proj_cn(h, w, bl, M, w.V, w.W, w.H1, s));
-      MARIE_TRY(cgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, Nb, p, M, mone, w.V, Nb, w.H1, M, one, w.W, Nb));
-      if (cgs_passes() > 1) {
+      const bool twice = cgs_passes() > 1;
+      MARIE_TRY(proj_cn(h, w, bl, M, w.V, w.W, w.H1, s, true));
+      MARIE_TRY(comb(w, bl, M, -1.f, w.V, w.H1, 1.f, w.W, s));
+      if (twice) {
         MARIE_TRY(proj_cn(h, w, bl, M, w.V, w.W, w.H2, s));
-        MARIE_TRY(cgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, Nb, p, M, mone, w.V, Nb, w.H2, M, one, w.W, Nb));
-      } else {
-        MARIE_CUDA_TRY(cudaMemsetAsync(w.H2, 0, sizeof(cplx<float>) * (size_t)M * p, s));
+        MARIE_TRY(comb(w, bl, M, -1.f, w.V, w.H2, 1.f, w.W, s));
+        MARIE_TRY(bio_move(h, bio_h2(p, mb), w.H2, (size_t)M * p * 8, true, s));
       }
       MARIE_TRY(bio_move(h, bio_h1(p, mb), w.H1, (size_t)M * p * 8, true, s));
-      MARIE_TRY(bio_move(h, bio_h2(p, mb), w.H2, (size_t)M * p * 8, true, s));
       if (prof.on) cudaEventRecord(prof.ev[2], s);
       MARIE_TRY(block_qr(h, w, bl, w.W, w.V + (int64_t)(j + 1) * p * Nb, Rq, s));   // synchronises
       if (prof.on) {
@@ -486,8 +507,8 @@ static marie_status bgmres_core(marie_vie* h, const std::vector<int>& cols, cons
       const cplx<float>* h2 = reinterpret_cast<const cplx<float>*>(h->bio + bio_h2(p, mb));
       for (int c = 0; c < p; ++c) {
         for (int64_t i = 0; i < M; ++i)
-          Hc[i + (size_t)rows * c] = zc((double)h1[i + M * c].x + h2[i + M * c].x,
-                                        (double)h1[i + M * c].y + h2[i + M * c].y);
+          Hc[i + (size_t)rows * c] = zc((double)h1[i + M * c].x + (twice ? h2[i + M * c].x : 0.f),
+                                        (double)h1[i + M * c].y + (twice ? h2[i + M * c].y : 0.f));
         for (int i = 0; i < p; ++i) Hc[M + i + (size_t)rows * c] = Rq[i + (size_t)p * c];
       }
       lsq.add_block(j, Hc, resid);
@@ -517,7 +538,7 @@ static marie_status bgmres_core(marie_vie* h, const std::vector<int>& cols, cons
     cplx<float>* up = reinterpret_cast<cplx<float>*>(h->bio + bio_up(p, mb));
     to_c64(Y, up);
     MARIE_TRY(bio_move(h, bio_up(p, mb), w.Sm, (size_t)n * p * 8, false, s));
-    MARIE_TRY(cgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, Nb, p, n, one, w.V, Nb, w.Sm, n, zero, w.W, Nb));
+    MARIE_TRY(comb(w, bl, n, 1.f, w.V, w.Sm, 0.f, w.W, s));
     k_add_block<<<vgrid(Nb, p), 256, 0, s>>>(x, Nb, w.W, Nb, w.map);
     MARIE_LAUNCH_CHECK();
     if (done || cyc + 1 == maxcyc) break;
@@ -526,7 +547,7 @@ static marie_status bgmres_core(marie_vie* h, const std::vector<int>& cols, cons
     MARIE_CUDA_TRY(cudaStreamSynchronize(s));     // the upload area held Y
     to_c64(Z, up);
     MARIE_TRY(bio_move(h, bio_up(p, mb), w.Sm, (size_t)(n + p) * p * 8, false, s));
-    MARIE_TRY(cgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, Nb, p, n + p, one, w.V, Nb, w.Sm, n + p, zero, w.W, Nb));
+    MARIE_TRY(comb(w, bl, n + p, 1.f, w.V, w.Sm, 0.f, w.W, s));
     MARIE_TRY(block_qr(h, w, bl, w.W, w.V, S0, s));
   }
   MARIE_CUDA_TRY(cudaStreamSynchronize(s));

@@ -115,13 +115,13 @@ __global__ void __launch_bounds__(256, 1) k4_z(MvArgs<T> a) {
     const int h = r & 1, r2 = r >> 1;
     const int b = r2 % NB, c = r2 / NB;
     const unsigned live = a.zq ? a.zq[b] : inside_bits(g3, NB, b);   // slices z = NB*q + b
-    const bool flip = (flips_of(e) >> c) & 1u;
+    const unsigned flip = (flips_of(e) >> c) << 31;
     cplx<T> u[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       cplx<T> val = (e < wl && ((live >> q) & 1u)) ? base[c * cstride + (int64_t)(NB * q + b) * row + e]
                                                    : cplx<T>{0, 0};
-      if (flip) val = cplx<T>{-val.x, -val.y};
+      val = flip_c(val, flip);
       if (h) val = val * a.az.tw2[NB * q + b];
       u[q] = val;
     }
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256, 1) k4_z(MvArgs<T> a) {
       for (int q = 0; q < 16; ++q) u[q] = mulc(u[q], a.az.tw2[NB * q + b]);
     }
     const bool st = act && e < wl;
-    const bool flip = (flips_of(e) >> c) & 1u;
+    const unsigned flip = (flips_of(e) >> c) << 31;
     const unsigned live = (a.zq ? a.zq[b] : inside_bits(g3, NB, b)) >> (8 * h);   // slices z = NB*(8h + j) + b
     cplx<T>* dst = base + c * cstride + (int64_t)(NB * 8 * h + b) * row + e;
 #pragma unroll
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256, 1) k4_z(MvArgs<T> a) {
       const cplx<T> send = h ? u[j] : u[8 + j];
       const cplx<T> recv = shfl_xor_c(send, W);
       const cplx<T> out = h ? recv + u[8 + j] : u[j] + recv;
-      if (st && ((live >> j) & 1u)) dst[(int64_t)NB * j * row] = flip ? cplx<T>{-out.x, -out.y} : out;
+      if (st && ((live >> j) & 1u)) dst[(int64_t)NB * j * row] = flip_c(out, flip);
     }
   }
 }

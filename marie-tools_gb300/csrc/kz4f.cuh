@@ -227,13 +227,13 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
     const int h = r & 1, r2 = r >> 1;
     const int b = r2 % NB, c = r2 / NB;
     const unsigned live = a.zq ? a.zq[b] : inside_bits(g3, NB, b);   // slices z = NB*q + b
-    const bool flip = (flips_of(e) >> c) & 1u;
+    const unsigned flip = (flips_of(e) >> c) << 31;
     ffc2 u[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       cplx<ff> val = (e < wl && ((live >> q) & 1u)) ? base[c * cstride + (int64_t)(NB * q + b) * row + e]
                                                     : cplx<ff>{ff(0), ff(0)};
-      if (flip) val = cplx<ff>{-val.x, -val.y};
+      val = flip_c(val, flip);
       if (h) val = val * a.az.tw2[NB * q + b];
       u[q] = to_ffc2(val);
     }
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
       for (int q = 0; q < 16; ++q) u[q] = mulc(u[q], a.az.tw2[NB * q + b]);
     }
     const bool st = act && e < wl;
-    const bool flip = (flips_of(e) >> c) & 1u;
+    const unsigned flip = (flips_of(e) >> c) << 31;
     const unsigned live = (a.zq ? a.zq[b] : inside_bits(g3, NB, b)) >> (8 * h);   // slices z = NB*(8h + j) + b
     cplx<ff>* dst = base + c * cstride + (int64_t)(NB * 8 * h + b) * row + e;
 #pragma unroll
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(256, 2) k4_zf(MvArgs<ff> a) {
       const cplx<ff> send = h ? u[j] : u[8 + j];
       const cplx<ff> recv = shfl_xor_c(send, W);
       const cplx<ff> out = h ? recv + u[8 + j] : u[j] + recv;
-      if (st && ((live >> j) & 1u)) dst[(int64_t)NB * j * row] = flip ? cplx<ff>{-out.x, -out.y} : out;
+      if (st && ((live >> j) & 1u)) dst[(int64_t)NB * j * row] = flip_c(out, flip);
     }
   }
 }

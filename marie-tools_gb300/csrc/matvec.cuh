@@ -156,6 +156,16 @@ __device__ __forceinline__ unsigned mirror_flips(bool mx, bool my) {
   return (mx ? mirror_mask<PWL>(0) : 0u) ^ (my ? mirror_mask<PWL>(1) : 0u);
 }
 
+// v with the sign bits flipped by mask (0 or 0x80000000).
+__device__ __forceinline__ cplx<double> flip_c(cplx<double> v, unsigned mask) {
+  const long long m = (long long)((unsigned long long)mask << 32);
+  return {__longlong_as_double(__double_as_longlong(v.x) ^ m), __longlong_as_double(__double_as_longlong(v.y) ^ m)};
+}
+__device__ __forceinline__ cplx<ff> flip_c(cplx<ff> v, unsigned mask) {
+  auto f = [mask](float x) { return __uint_as_float(__float_as_uint(x) ^ mask); };
+  return {ff(f(v.x.hi), f(v.x.lo)), ff(f(v.y.hi), f(v.y.lo))};
+}
+
 // Body-vector output of the modes other than MV_GRID for component c, body
 // voxel s and right-hand side rhs, given v = (operator x) at that voxel.
 template <typename T>
