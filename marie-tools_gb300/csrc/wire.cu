@@ -23,6 +23,7 @@
 #include <cmath>
 #include <vector>
 
+#include "fp64math.cuh"
 #include "internal.h"
 
 namespace marie {
@@ -78,16 +79,17 @@ __global__ void __launch_bounds__(128) k_wire(const int64_t* __restrict__ idxS, 
             const WireSrc q = tile[i];
             const double rx = px - q.x, ry = py - q.y, rz = pz - q.z;
             const double R2 = rx * rx + ry * ry + rz * rz;
-            const double R = sqrt(R2);
+            double R;
+            const double iR = inv_sqrt(R2, R), iR2 = iR * iR;
             const double kR = k0 * R;
             double sn, cs;
-            sincos(kR, &sn, &cs);
-            const double iR3 = 1.0 / (R2 * R);
+            sin_cos(kR, &sn, &cs);
+            const double iR3 = iR2 * iR;
             // kappa = e^{-ikR}/R^3
             const double kr = cs * iR3, ki = -sn * iR3;
             if constexpr (KIND == 0) {
               // P = (k^2 R^2 - 3 - 3i kR)/R^2; c2 = k^2 R^2 - 1 - i kR
-              const double Pr = (k2 * R2 - 3.0) / R2, Pi = -3.0 * kR / R2;
+              const double Pr = (k2 * R2 - 3.0) * iR2, Pi = -3.0 * kR * iR2;
               const double c2r = k2 * R2 - 1.0, c2i = -kR;
               // R.J (complex)
               const double dr = rx * q.jxr + ry * q.jyr + rz * q.jzr;
