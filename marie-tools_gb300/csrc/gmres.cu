@@ -27,6 +27,16 @@ typedef cplx<double> zd;
 constexpr int kVT = 256;          // threads per vector CTA
 constexpr int kVE = 8;            // elements per thread
 constexpr int kCH = kVT * kVE;    // elements per chunk
+// Short vectors: one element per thread and CTAs of 64, so that the FP64 work (two
+// FMAs per clock and SM) spreads over the chip.  32^3 PWC sphere, complex128, 83
+// steps: 26.2 -> 11.9 ms a solve, together with k_givens and k_solve_y by warps and
+// the norm summed where it scales.  The rule looks at one vector alone, so that a
+// solve in a batch sums in the order of a single one; 30312 unknowns, one
+// right-hand side, 21.5 -> 9.1 ms; 121248, eight, 242 -> 240; with 231456, eight,
+// it would be 85 -> 99.
+constexpr int kVTS = 64;
+constexpr int kDotVE = 4;         // elements per thread of their projections (a reduction costs as much as four)
+static bool short_vectors(int64_t Nb) { return (Nb + kCH - 1) / kCH <= 64; }
 
 enum RhsState : int { ST_ACTIVE = 0, ST_DONE = 1, ST_MAXIT = 2, ST_NONFINITE = 3 };
 
@@ -61,8 +71,9 @@ __device__ __forceinline__ cplx<A> block_sum(cplx<A> v, cplx<A>* sh) {
 template <typename T>
 struct Acc { typedef T type; };
 
-// part[(r*(m+1) + j)*nch + chunk] = sum_i conj(V_j[i]) w[i], j in [0, k]
-template <typename T>
+// part[(r*(m+1) + j)*nch + chunk] = sum_i conj(V_j[i]) w[i], j in [0, k]; the
+// CTAs of a chunk (gridDim.z) take the j in turn
+template <typename T, int VT, int VE>
 __global__ void k_dots(const cplx<T>* V, int64_t ld, int64_t Nb, int k, int mp1, const unsigned char* act,
                        zd* part, int nch) {
   typedef typename Acc<T>::type A;
@@ -72,19 +83,19 @@ __global__ void k_dots(const cplx<T>* V, int64_t ld, int64_t Nb, int k, int mp1,
   const int chunk = blockIdx.x;
   const cplx<T>* base = V + (int64_t)r * mp1 * ld;
   const cplx<T>* w = base + (int64_t)(k + 1) * ld;
-  cplx<T> wv[kVE];
-  const int64_t i0 = (int64_t)chunk * kCH + threadIdx.x;
+  cplx<T> wv[VE];
+  const int64_t i0 = (int64_t)chunk * (VT * VE) + threadIdx.x;
 #pragma unroll
-  for (int e = 0; e < kVE; ++e) {
-    const int64_t i = i0 + (int64_t)e * kVT;
+  for (int e = 0; e < VE; ++e) {
+    const int64_t i = i0 + (int64_t)e * VT;
     wv[e] = i < Nb ? w[i] : cplx<T>{0, 0};
   }
-  for (int j = 0; j <= k; ++j) {
+  for (int j = blockIdx.z; j <= k; j += gridDim.z) {
     const cplx<T>* vj = base + (int64_t)j * ld;
     cplx<A> acc = {0, 0};
 #pragma unroll
-    for (int e = 0; e < kVE; ++e) {
-      const int64_t i = i0 + (int64_t)e * kVT;
+    for (int e = 0; e < VE; ++e) {
+      const int64_t i = i0 + (int64_t)e * VT;
       if (i < Nb) {
         const cplx<T> v = vj[i];
         acc.x += (A)v.x * (A)wv[e].x + (A)v.y * (A)wv[e].y;
@@ -122,7 +133,7 @@ __global__ void k_reduce_dots(const zd* part, int nch, int k, int mp1, int m, co
 }
 
 // w -= sum_j V_j h_j ; npart[r*nch + chunk] = ||w_chunk||^2
-template <typename T>
+template <typename T, int VT, int VE>
 __global__ void k_update(cplx<T>* V, int64_t ld, int64_t Nb, int k, int mp1, int m, const unsigned char* act,
                          const zd* H, double* npart, int nch) {
   typedef typename Acc<T>::type A;
@@ -138,19 +149,20 @@ __global__ void k_update(cplx<T>* V, int64_t ld, int64_t Nb, int k, int mp1, int
   __syncthreads();
   cplx<T>* base = V + (int64_t)r * mp1 * ld;
   cplx<T>* w = base + (int64_t)(k + 1) * ld;
-  const int64_t i0 = (int64_t)chunk * kCH + threadIdx.x;
-  cplx<T> wv[kVE];
+  const int64_t i0 = (int64_t)chunk * (VT * VE) + threadIdx.x;
+  cplx<T> wv[VE];
 #pragma unroll
-  for (int e = 0; e < kVE; ++e) {
-    const int64_t i = i0 + (int64_t)e * kVT;
+  for (int e = 0; e < VE; ++e) {
+    const int64_t i = i0 + (int64_t)e * VT;
     wv[e] = i < Nb ? w[i] : cplx<T>{0, 0};
   }
+#pragma unroll (VE == 1 ? 8 : 1)
   for (int j = 0; j <= k; ++j) {
     const cplx<T>* vj = base + (int64_t)j * ld;
     const cplx<T> hj = hs[j];
 #pragma unroll
-    for (int e = 0; e < kVE; ++e) {
-      const int64_t i = i0 + (int64_t)e * kVT;
+    for (int e = 0; e < VE; ++e) {
+      const int64_t i = i0 + (int64_t)e * VT;
       if (i < Nb) {
         const cplx<T> v = vj[i];
         wv[e].x -= v.x * hj.x - v.y * hj.y;
@@ -160,8 +172,8 @@ __global__ void k_update(cplx<T>* V, int64_t ld, int64_t Nb, int k, int mp1, int
   }
   A nrm = 0;
 #pragma unroll
-  for (int e = 0; e < kVE; ++e) {
-    const int64_t i = i0 + (int64_t)e * kVT;
+  for (int e = 0; e < VE; ++e) {
+    const int64_t i = i0 + (int64_t)e * VT;
     if (i < Nb) {
       w[i] = wv[e];
       nrm += (A)wv[e].x * (A)wv[e].x + (A)wv[e].y * (A)wv[e].y;
@@ -172,18 +184,18 @@ __global__ void k_update(cplx<T>* V, int64_t ld, int64_t Nb, int k, int mp1, int
 }
 
 // npart[r*nch + chunk] = ||v_r chunk||^2 for v_r = base + r*rs
-template <typename T>
+template <typename T, int VT, int VE>
 __global__ void k_norm2(const cplx<T>* v, int64_t rs, int64_t Nb, const unsigned char* act, double* npart, int nch) {
   typedef typename Acc<T>::type A;
   __shared__ cplx<A> sh[32];
   const int r = blockIdx.y;
   if (act && !act[r]) return;
   const cplx<T>* p = v + (int64_t)r * rs;
-  const int64_t i0 = (int64_t)blockIdx.x * kCH + threadIdx.x;
+  const int64_t i0 = (int64_t)blockIdx.x * (VT * VE) + threadIdx.x;
   A nrm = 0;
 #pragma unroll
-  for (int e = 0; e < kVE; ++e) {
-    const int64_t i = i0 + (int64_t)e * kVT;
+  for (int e = 0; e < VE; ++e) {
+    const int64_t i = i0 + (int64_t)e * VT;
     if (i < Nb) {
       const cplx<T> x = p[i];
       nrm += (A)x.x * (A)x.x + (A)x.y * (A)x.y;
@@ -218,6 +230,32 @@ __global__ void k_scale(cplx<T>* v, int64_t rs, int64_t Nb, const unsigned char*
     p[i] = scale(p[i], inv);
 }
 
+// k_reduce_norm and k_scale in one launch for short vectors: every CTA sums the
+// rhs' partials in the same fixed order, the first writes the norm.
+template <typename T>
+__global__ void __launch_bounds__(256) k_norm_scale(cplx<T>* v, int64_t rs, int64_t Nb, const unsigned char* act,
+                                                    const double* npart, int nch, double* out) {
+  __shared__ double sv;
+  const int r = blockIdx.y;
+  if (!act[r]) return;
+  if (threadIdx.x < 32) {
+    const double* p = npart + (int64_t)r * nch;
+    double s = 0;
+    for (int c = threadIdx.x; c < nch; c += 32) s += p[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) {
+      sv = sqrt(s);
+      if (blockIdx.x == 0) out[r] = sv;
+    }
+  }
+  __syncthreads();
+  const T inv = sv > 0 ? (T)(1.0 / sv) : (T)0;
+  cplx<T>* p = v + (int64_t)r * rs;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < Nb; i += (int64_t)gridDim.x * blockDim.x)
+    p[i] = scale(p[i], inv);
+}
+
 struct GmState {
   zd* H;          // [nrhs][(m+1)*m]   Hessenberg (original)
   zd* R;          // [nrhs][(m+1)*m]   rotated copy
@@ -237,10 +275,15 @@ struct GmState {
   double* npart;  // [nrhs][nch]
 };
 
-// Givens step for column k (one thread per rhs).  Sets incyc=0 when the cycle
-// ends (converged, breakdown, k+1 == m or non-finite).
-__global__ void k_givens(GmState st, int k, int m, int nrhs) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// Givens step for column k, one warp per rhs: the column and the rotations in
+// shared memory, each rotation's four real results in four lanes (an FP64
+// instruction occupies a scheduler for 64 clocks however few lanes it serves:
+// three per rotation instead of twelve).  Sets incyc=0 when the cycle ends
+// (converged, breakdown, k+1 == m or non-finite).
+__global__ void __launch_bounds__(32) k_givens(GmState st, int k, int m, int nrhs) {
+  __shared__ zd col[kMaxRestart + 1], ssn[kMaxRestart];
+  __shared__ double scs[kMaxRestart];
+  const int r = blockIdx.x, lane = threadIdx.x;
   if (r >= nrhs || !st.incyc[r]) return;
   const int mp1 = m + 1;
   zd* H = st.H + (int64_t)r * mp1 * m;
@@ -249,51 +292,68 @@ __global__ void k_givens(GmState st, int k, int m, int nrhs) {
   zd* sn = st.sn + (int64_t)r * m;
   zd* g = st.g + (int64_t)r * mp1;
   const double hk1 = st.hnorm[r];
-  H[k + 1 + mp1 * k] = zd{hk1, 0};
-  for (int i = 0; i <= k; ++i) R[i + mp1 * k] = H[i + mp1 * k];
-  R[k + 1 + mp1 * k] = zd{hk1, 0};
-  for (int i = 0; i < k; ++i) {
-    const zd a = R[i + mp1 * k], b = R[i + 1 + mp1 * k];
-    const double c = cs[i];
-    const zd s = sn[i];
-    R[i + mp1 * k] = zd{c * a.x + (s.x * b.x - s.y * b.y), c * a.y + (s.x * b.y + s.y * b.x)};
-    // -conj(s)*a + c*b
-    R[i + 1 + mp1 * k] = zd{-(s.x * a.x + s.y * a.y) + c * b.x, -(s.x * a.y - s.y * a.x) + c * b.y};
+  for (int i = lane; i <= k; i += 32) col[i] = H[i + mp1 * k];
+  for (int i = lane; i < k; i += 32) {
+    scs[i] = cs[i];
+    ssn[i] = sn[i];
   }
-  const zd a = R[k + mp1 * k];
-  const double b = hk1;
-  const double na = sqrt(a.x * a.x + a.y * a.y);
-  double c;
-  zd s;
-  if (na == 0.0) {
-    c = 0.0;
-    s = zd{1.0, 0.0};
-  } else {
-    const double t = sqrt(na * na + b * b);
-    c = na / t;
-    s = zd{a.x / na * b / t, a.y / na * b / t};
+  __syncwarp();
+  // rotation i on (a, b = col[i+1]):  col[i] = c a + s b,  a = -conj(s) a + c b
+  zd a = col[0];
+  {
+    const bool im = lane & 1, lower = lane & 2;
+    for (int i = 0; i < k; ++i) {
+      const zd b = col[i + 1], s = ssn[i];
+      const double c = scs[i];
+      const double bq = im ? b.y : b.x, bo = im ? b.x : b.y;       // the lane's part of b and the other
+      const double aq = im ? a.y : a.x, ao = im ? a.x : a.y;
+      const double sy = im ? s.y : -s.y;
+      // upper: c a + s.x b + (-+ s.y) b';  lower: c b - s.x a + (-+ s.y) a'
+      double t = sy * (lower ? ao : bo);
+      t = fma(lower ? -s.x : s.x, lower ? aq : bq, t);
+      t = fma(c, lower ? bq : aq, t);
+      const double ux = __shfl_sync(0xffffffffu, t, 0), uy = __shfl_sync(0xffffffffu, t, 1);
+      a = zd{__shfl_sync(0xffffffffu, t, 2), __shfl_sync(0xffffffffu, t, 3)};
+      if (lane == 0) col[i] = zd{ux, uy};
+    }
   }
-  cs[k] = c;
-  sn[k] = s;
-  R[k + mp1 * k] = zd{c * a.x + s.x * b, c * a.y + s.y * b};
-  R[k + 1 + mp1 * k] = zd{0, 0};
-  const zd gk = g[k];
-  g[k + 1] = zd{-(s.x * gk.x + s.y * gk.y), -(s.x * gk.y - s.y * gk.x)};
-  g[k] = zd{c * gk.x, c * gk.y};
-  const double res = sqrt(g[k + 1].x * g[k + 1].x + g[k + 1].y * g[k + 1].y);
-  st.resid[r] = res;
-  st.hist[(int64_t)r * m + k] = res;
-  st.kr[r] = k + 1;
-  if (!isfinite(res) || !isfinite(hk1)) {
-    st.incyc[r] = 0;
-    return;
+  if (lane == 0) {
+    const double b = hk1;
+    const double na = sqrt(a.x * a.x + a.y * a.y);
+    double c;
+    zd s;
+    if (na == 0.0) {
+      c = 0.0;
+      s = zd{1.0, 0.0};
+    } else {
+      const double t = sqrt(na * na + b * b);
+      c = na / t;
+      s = zd{a.x / na * b / t, a.y / na * b / t};
+    }
+    cs[k] = c;
+    sn[k] = s;
+    col[k] = zd{c * a.x + s.x * b, c * a.y + s.y * b};
+    H[k + 1 + mp1 * k] = zd{hk1, 0};
+    R[k + 1 + mp1 * k] = zd{0, 0};
+    const zd gk = g[k];
+    const zd g1 = zd{-(s.x * gk.x + s.y * gk.y), -(s.x * gk.y - s.y * gk.x)};
+    g[k + 1] = g1;
+    g[k] = zd{c * gk.x, c * gk.y};
+    const double res = sqrt(g1.x * g1.x + g1.y * g1.y);
+    st.resid[r] = res;
+    st.hist[(int64_t)r * m + k] = res;
+    st.kr[r] = k + 1;
+    if (!isfinite(res) || !isfinite(hk1) || res < st.tolabs[r] || k + 1 == m || hk1 == 0.0) st.incyc[r] = 0;
   }
-  if (res < st.tolabs[r] || k + 1 == m || hk1 == 0.0) st.incyc[r] = 0;
+  __syncwarp();
+  for (int i = lane; i <= k; i += 32) R[i + mp1 * k] = col[i];
 }
 
-// y = R^{-1} g (k x k), res = beta e1 - H y ((k+1) entries); one thread per rhs.
-__global__ void k_solve_y(GmState st, int m, int nrhs, const unsigned char* ran) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// y = R^{-1} g (k x k), res = beta e1 - H y ((k+1) entries); one warp per rhs,
+// lanes own rows (columns of R and H are read coalesced).
+__global__ void __launch_bounds__(32) k_solve_y(GmState st, int m, int nrhs, const unsigned char* ran) {
+  constexpr int kRows = kMaxRestart / 32 + 1;
+  const int r = blockIdx.x, lane = threadIdx.x;
   if (r >= nrhs || !ran[r]) return;
   const int k = st.kr[r];
   const int mp1 = m + 1;
@@ -302,17 +362,37 @@ __global__ void k_solve_y(GmState st, int m, int nrhs, const unsigned char* ran)
   const zd* g = st.g + (int64_t)r * mp1;
   zd* y = st.y + (int64_t)r * m;
   zd* res = st.res + (int64_t)r * mp1;
+  __shared__ zd ys[kMaxRestart];
+  zd acc[kRows];
+#pragma unroll
+  for (int q = 0; q < kRows; ++q) acc[q] = lane + 32 * q < k ? g[lane + 32 * q] : zd{0, 0};
   for (int i = k - 1; i >= 0; --i) {
-    zd acc = g[i];
-    for (int j = i + 1; j < k; ++j) acc = acc - R[i + mp1 * j] * y[j];
-    const zd d = R[i + mp1 * i];
+    zd col[kRows];
+#pragma unroll
+    for (int q = 0; q < kRows; ++q)
+      if (32 * q <= i) col[q] = lane + 32 * q <= i ? R[lane + 32 * q + mp1 * i] : zd{0, 0};
+    zd v{0, 0}, d{0, 0};
+#pragma unroll
+    for (int q = 0; q < kRows; ++q)
+      if (lane + 32 * q == i) {
+        v = acc[q];
+        d = col[q];
+      }
     const double dd = d.x * d.x + d.y * d.y;
-    y[i] = dd > 0 ? zd{(acc.x * d.x + acc.y * d.y) / dd, (acc.y * d.x - acc.x * d.y) / dd} : zd{0, 0};
+    zd yi = dd > 0 ? zd{(v.x * d.x + v.y * d.y) / dd, (v.y * d.x - v.x * d.y) / dd} : zd{0, 0};
+    yi.x = __shfl_sync(0xffffffffu, yi.x, i & 31);
+    yi.y = __shfl_sync(0xffffffffu, yi.y, i & 31);
+    if (lane == 0) ys[i] = yi;
+#pragma unroll
+    for (int q = 0; q < kRows; ++q)
+      if (32 * q < i && lane + 32 * q < i) acc[q] = acc[q] - col[q] * yi;
   }
-  for (int i = 0; i <= k; ++i) {
-    zd acc = i == 0 ? zd{st.beta[r], 0} : zd{0, 0};
-    for (int j = 0; j < k; ++j) acc = acc - H[i + mp1 * j] * y[j];
-    res[i] = acc;
+  __syncwarp();
+  for (int i = lane; i < k; i += 32) y[i] = ys[i];
+  for (int i = lane; i <= k; i += 32) {
+    zd a = i == 0 ? zd{st.beta[r], 0} : zd{0, 0};
+    for (int j = 0; j < k; ++j) a = a - H[i + mp1 * j] * ys[j];
+    res[i] = a;
   }
 }
 
@@ -648,7 +728,14 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
                                std::vector<RhsLog>& log, int* matvecs, cudaStream_t s, Scratch& sc) {
   const int64_t Nb = h->Nb;
   const int mp1 = m + 1;
-  const int nch = (int)((Nb + kCH - 1) / kCH);
+  const bool brief = short_vectors(Nb);
+  const int per = brief ? kVTS : kCH;
+  const int nch = (int)((Nb + per - 1) / per);
+  const int nchd = brief ? (int)((Nb + kVTS * kDotVE - 1) / (kVTS * kDotVE)) : nch;   // of the projections
+  // CTAs per chunk in the projections of short vectors
+  auto jsplit = [&](int k) {
+    return (unsigned)(brief ? std::max(1, std::min(k + 1, (int)(2048 / std::max<int64_t>(1, (int64_t)nchd * nrhs)))) : 1);
+  };
   GmState st;
   MARIE_TRY(sc.get(&st.H, (size_t)nrhs * mp1 * m));
   MARIE_TRY(sc.get(&st.R, (size_t)nrhs * mp1 * m));
@@ -678,8 +765,12 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
   const int64_t vrs = (int64_t)mp1 * Nb;
   const dim3 cg((unsigned)nch, (unsigned)nrhs);
   const unsigned sb = (unsigned)((nrhs + 127) / 128);
+  auto norm2 = [&](const cplx<T>* v) {
+    if (brief) k_norm2<T, kVTS, 1><<<cg, kVTS, 0, s>>>(v, vrs, Nb, d_mask, st.npart, nch);
+    else k_norm2<T, kVT, kVE><<<cg, kVT, 0, s>>>(v, vrs, Nb, d_mask, st.npart, nch);
+  };
   // beta = ||r0||
-  k_norm2<T><<<cg, kVT, 0, s>>>(V, vrs, Nb, d_mask, st.npart, nch);
+  norm2(V);
   MARIE_LAUNCH_CHECK();
   k_reduce_norm<<<(nrhs + 7) / 8, 256, 0, s>>>(st.npart, nch, nrhs, d_mask, st.beta);
   MARIE_LAUNCH_CHECK();
@@ -717,18 +808,27 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
         for (int k = k0; k < k1; ++k) {
           MARIE_TRY(launch_matvec<T>(h, sc.adjoint ? MV_VIE_ADJ : MV_VIE, sc.adjoint ? OP_N_ADJ : OP_N,
                                      V + (int64_t)k * ld, vrs, V + (int64_t)(k + 1) * ld, vrs, nrhs, st.incyc, q));
-          k_dots<T><<<cg, kVT, 0, q>>>(V, ld, Nb, k, mp1, st.incyc, st.part, nch);
+          const dim3 dg((unsigned)nchd, (unsigned)nrhs, jsplit(k));
+          if (brief) k_dots<T, kVTS, kDotVE><<<dg, kVTS, 0, q>>>(V, ld, Nb, k, mp1, st.incyc, st.part, nchd);
+          else k_dots<T, kVT, kVE><<<dg, kVT, 0, q>>>(V, ld, Nb, k, mp1, st.incyc, st.part, nchd);
           MARIE_LAUNCH_CHECK();
-          k_reduce_dots<<<dim3((k + 8) / 8, nrhs), 256, 0, q>>>(st.part, nch, k, mp1, m, st.incyc, st.H);
+          k_reduce_dots<<<dim3((k + 8) / 8, nrhs), 256, 0, q>>>(st.part, nchd, k, mp1, m, st.incyc, st.H);
           MARIE_LAUNCH_CHECK();
-          k_update<T><<<cg, kVT, 0, q>>>(V, ld, Nb, k, mp1, m, st.incyc, st.H, st.npart, nch);
-          MARIE_LAUNCH_CHECK();
-          k_reduce_norm<<<(nrhs + 7) / 8, 256, 0, q>>>(st.npart, nch, nrhs, st.incyc, st.hnorm);
+          if (brief) k_update<T, kVTS, 1><<<cg, kVTS, 0, q>>>(V, ld, Nb, k, mp1, m, st.incyc, st.H, st.npart, nch);
+          else k_update<T, kVT, kVE><<<cg, kVT, 0, q>>>(V, ld, Nb, k, mp1, m, st.incyc, st.H, st.npart, nch);
           MARIE_LAUNCH_CHECK();
           // scale with the mask before the Givens step clears finished rhs
-          k_scale<T><<<vgrid(Nb, nrhs), 256, 0, q>>>(V + (int64_t)(k + 1) * ld, vrs, Nb, st.incyc, st.hnorm);
-          MARIE_LAUNCH_CHECK();
-          k_givens<<<sb, 128, 0, q>>>(st, k, m, nrhs);
+          if (brief) {
+            k_norm_scale<T><<<vgrid(Nb, nrhs), 256, 0, q>>>(V + (int64_t)(k + 1) * ld, vrs, Nb, st.incyc, st.npart, nch,
+                                                            st.hnorm);
+            MARIE_LAUNCH_CHECK();
+          } else {
+            k_reduce_norm<<<(nrhs + 7) / 8, 256, 0, q>>>(st.npart, nch, nrhs, st.incyc, st.hnorm);
+            MARIE_LAUNCH_CHECK();
+            k_scale<T><<<vgrid(Nb, nrhs), 256, 0, q>>>(V + (int64_t)(k + 1) * ld, vrs, Nb, st.incyc, st.hnorm);
+            MARIE_LAUNCH_CHECK();
+          }
+          k_givens<<<nrhs, 32, 0, q>>>(st, k, m, nrhs);
           MARIE_LAUNCH_CHECK();
         }
         MARIE_TRY(chan_get(h, SLOT_INCYC, nrhs, st.incyc, nrhs, q));
@@ -761,13 +861,13 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
     // finalize the cycle of every rhs that ran it
     MARIE_TRY(chan_get(h, SLOT_KR, nrhs, st.kr, nrhs * sizeof(int), s));
     MARIE_TRY(chan_put(h, SLOT_MASK, nrhs, d_mask, start.data(), nrhs, s));
-    k_solve_y<<<sb, 128, 0, s>>>(st, m, nrhs, d_mask);
+    k_solve_y<<<nrhs, 32, 0, s>>>(st, m, nrhs, d_mask);
     MARIE_LAUNCH_CHECK();
     k_xupdate<T><<<vgrid(Nb, nrhs), 256, 0, s>>>(V, ld, mp1, m, Nb, d_mask, st, x, Nb);
     MARIE_LAUNCH_CHECK();
     k_rform<T><<<vgrid(Nb, nrhs), 256, 0, s>>>(V, ld, mp1, Nb, d_mask, st);
     MARIE_LAUNCH_CHECK();
-    k_norm2<T><<<cg, kVT, 0, s>>>(V, vrs, Nb, d_mask, st.npart, nch);
+    norm2(V);
     MARIE_LAUNCH_CHECK();
     k_reduce_norm<<<(nrhs + 7) / 8, 256, 0, s>>>(st.npart, nch, nrhs, d_mask, st.beta);
     MARIE_LAUNCH_CHECK();
@@ -806,7 +906,7 @@ static marie_status true_residual(marie_vie* h, int nrhs, const zd* b, const zd*
   ++*matvecs;
   k_residual<<<vgrid(Nb, nrhs), 256, 0, s>>>(b, r, Nb, d_mask);
   MARIE_LAUNCH_CHECK();
-  k_norm2<double><<<dim3(nch, nrhs), kVT, 0, s>>>((const cplx<double>*)r, Nb, Nb, d_mask, npart, nch);
+  k_norm2<double, kVT, kVE><<<dim3(nch, nrhs), kVT, 0, s>>>((const cplx<double>*)r, Nb, Nb, d_mask, npart, nch);
   MARIE_LAUNCH_CHECK();
   k_reduce_norm<<<(nrhs + 7) / 8, 256, 0, s>>>(npart, nch, nrhs, d_mask, nr);
   MARIE_LAUNCH_CHECK();
@@ -826,7 +926,7 @@ static marie_status norms(marie_vie* h, int nrhs, const zd* v, std::vector<doubl
   double *npart = nullptr, *nr = nullptr;
   MARIE_TRY(sc.get(&npart, (size_t)nrhs * nch));
   MARIE_TRY(sc.get(&nr, nrhs));
-  k_norm2<double><<<dim3(nch, nrhs), kVT, 0, s>>>((const cplx<double>*)v, Nb, Nb, nullptr, npart, nch);
+  k_norm2<double, kVT, kVE><<<dim3(nch, nrhs), kVT, 0, s>>>((const cplx<double>*)v, Nb, Nb, nullptr, npart, nch);
   MARIE_LAUNCH_CHECK();
   k_reduce_norm<<<(nrhs + 7) / 8, 256, 0, s>>>(npart, nch, nrhs, nullptr, nr);
   MARIE_LAUNCH_CHECK();
