@@ -132,6 +132,27 @@ static void digit_maps(const FftPlan& pl, std::vector<int>& kofp, std::vector<in
   }
 }
 
+// c + i s of modulus one in float-float.  Of the low parts next to the exact ones
+// the pair that keeps the modulus nearest one: a modulus error is the same in every
+// product and adds up over the transforms, a phase error takes itself back in the
+// inverse ones.
+static cplx<ff> unit_ff(double c, double s) {
+  const float hc = (float)c, hs = (float)s;
+  const float lc = (float)(c - (double)hc), ls = (float)(s - (double)hs);
+  cplx<ff> best{ff(hc, lc), ff(hs, ls)};
+  auto modulus = [&](float a, float b) {
+    return std::abs(c * (((double)hc - c) + (double)a) + s * (((double)hs - s) + (double)b));
+  };
+  if (lc == 0.0f || ls == 0.0f) return best;   // an axis or diagonal value that needs no low part
+  for (int i = -1; i <= 1; ++i)
+    for (int j = -1; j <= 1; ++j) {
+      const float a = i ? std::nextafterf(lc, i * INFINITY) : lc, b = j ? std::nextafterf(ls, j * INFINITY) : ls;
+      const double phase = std::abs(c * (((double)hs - s) + (double)b) - s * (((double)hc - c) + (double)a));
+      if (phase < 2e-15 && modulus(a, b) < modulus(best.x.lo, best.y.lo)) best = cplx<ff>{ff(hc, a), ff(hs, b)};
+    }
+  return best;
+}
+
 template <typename T>
 static marie_status build_axis(marie_vie* h, int n, AxisDev<T>& ax) {
   if (!make_plan(n, &ax.plan)) {
@@ -144,6 +165,7 @@ static marie_status build_axis(marie_vie* h, int n, AxisDev<T>& ax) {
     const long double b = a / 2.0L;
     tw[k] = cplx<T>{prec_from<T>(std::cos(a)), prec_from<T>(std::sin(a))};
     tw2[k] = cplx<T>{prec_from<T>(std::cos(b)), prec_from<T>(std::sin(b))};
+    if constexpr (std::is_same<T, ff>::value) tw2[k] = unit_ff((double)std::cos(b), (double)std::sin(b));
   }
   std::vector<int> kofp, pofk;
   digit_maps(ax.plan, kofp, pofk);

@@ -13,22 +13,29 @@ namespace marie {
 __host__ __device__ constexpr int kz4_stride(int N, int W) { return N + (W >= 16 ? 1 : 16 / W); }
 __host__ __device__ constexpr int kz4_halfpad(int W) { return W >= 16 ? 0 : 8 / W; }
 
+// Float-float x and y passes (xy4f.cuh): twiddles (32 bytes each), sequence stride
+// in 16-byte elements, and shared memory of a tile of w lines.
+__host__ __device__ constexpr int xyf_tw(int n) { return 31 * (n / 16); }
+__host__ __device__ constexpr int xyf_stride(int n) { return n + 5; }
+__host__ __device__ constexpr size_t xyf_smem(int n, int w) {
+  return (size_t)32 * xyf_tw(n) + (size_t)2 * w * xyf_stride(n) * 16;
+}
+
 // Sequence stride of k4_zp (complex64, packed pairs) in 16-byte pairs.
 __host__ __device__ constexpr int kzp_stride(int N, int W) { return N + (W >= 4 ? 2 : 8 / W); }
-// k4_zf (float-float, 16-byte elements): the same stride and an odd-half pad
-// of 4/W, which put the eight lanes of every quarter-warp of its five phases
-// on distinct 16-byte bank groups (checked by enumerating lane addresses).
-__host__ __device__ constexpr int kzf_stride(int N, int W) { return N + (W >= 8 ? 1 : 8 / W); }
-__host__ __device__ constexpr int kzf_halfpad(int W) { return W >= 8 ? 0 : 4 / W; }
+// k4_zf (float-float, 16-byte elements): sequence stride, and pad of a quarter of
+// a sequence, per tile width (with eight elements or more those alone spread).
+__host__ __device__ constexpr int kzf_stride(int N, int W) { return N + (W >= 8 ? 1 : W == 4 ? 6 : W == 2 ? 4 : 3); }
+__host__ __device__ constexpr int kzf_pad(int W) { return W >= 8 ? 0 : 1; }
 
 // Shared-memory bytes of the z pass: k4_z (native complex128: twiddles +
-// both halves), k4_zf (float-float: 32-byte twiddle entries + both halves)
+// both halves), k4_zf (float-float: twiddles of 32 bytes + both halves)
 // or k4_zp (complex64: twiddle tables, slice masks, tile elements, pairs).
 template <typename T>
 __host__ inline size_t kz4_smem(int N, int C, int W) {
   const size_t NB = N / 16;
   if (sizeof(T) == 4) return 272 * NB + 64 + 544 + (size_t)C * W * kzp_stride(N, W) * 16;
-  if (std::is_same<T, ff>::value) return (36 * NB + 2 * (size_t)C * W * kzf_stride(N, W) + kzf_halfpad(W)) * 16;
+  if (std::is_same<T, ff>::value) return (size_t)32 * xyf_tw(N) + 2 * (size_t)C * W * kzf_stride(N, W) * 16;
   const size_t half = (size_t)C * W * kz4_stride(N, W);
   return (N + 2 * half + kz4_halfpad(W)) * sizeof(cplx<T>);
 }
@@ -105,8 +112,11 @@ marie_status launch_fast_chunk(marie_vie* h, int op, MvArgs<T>& a, int nb, cudaS
   const int n1 = a.n1, n2 = a.n2, n3 = a.n3, C = h->C;
   const size_t sz = sizeof(cplx<T>);
   constexpr bool c64 = std::is_same<T, float>::value;
-  const size_t smx = (size_t)(n1 + (size_t)2 * a.TY * a.R * (n1 + 1)) * sz;
-  const size_t smy = (size_t)(n2 + (size_t)2 * (c64 ? a.TZY : a.TXY) * a.R * (n2 + 1)) * sz;
+  auto smxy = [&](int n, int w) {
+    return std::is_same<T, ff>::value ? xyf_smem(n, w) : (n + (size_t)2 * w * (n + 1)) * sz;
+  };
+  const size_t smx = smxy(n1, a.TY * a.R);
+  const size_t smy = smxy(n2, (c64 ? a.TZY : a.TXY) * a.R);
   const size_t smz = kz4_smem<T>(n3, C, a.TX * a.R);
   // x: TY rows (complex64: slices) per tile; y: TXY kx of a row (complex64: TZY slices)
   dim3 gx(c64 ? (a.g3 + a.TY - 1) / a.TY : (a.g2 + a.TY - 1) / a.TY, c64 ? a.g2 : a.g3, nb * C);

@@ -24,6 +24,14 @@ static void launch_x(bool inv, const MvArgs<T>& a, dim3 g, size_t smem, cudaStre
       smem_opt_in(k4c_inv_x<NB>, oi);
       k4c_inv_x<NB><<<g, 256, smem, s>>>(a);
     }
+  } else if constexpr (std::is_same<T, ff>::value) {
+    if (!inv) {
+      smem_opt_in(k4f_fwd_x<NB>, of);
+      k4f_fwd_x<NB><<<g, 256, smem, s>>>(a);
+    } else {
+      smem_opt_in(k4f_inv_x<NB>, oi);
+      k4f_inv_x<NB><<<g, 256, smem, s>>>(a);
+    }
   } else if (!inv) {
     smem_opt_in(k4_fwd_x<T, NB>, of);
     k4_fwd_x<T, NB><<<g, 256, smem, s>>>(a);
@@ -44,6 +52,14 @@ static void launch_y(bool inv, const MvArgs<T>& a, dim3 g, size_t smem, cudaStre
       smem_opt_in(k4c_inv_y<NB>, oi);
       k4c_inv_y<NB><<<g, 256, smem, s>>>(a);
     }
+  } else if constexpr (std::is_same<T, ff>::value) {
+    if (!inv) {
+      smem_opt_in(k4f_fwd_y<NB>, of);
+      k4f_fwd_y<NB><<<g, 256, smem, s>>>(a);
+    } else {
+      smem_opt_in(k4f_inv_y<NB>, oi);
+      k4f_inv_y<NB><<<g, 256, smem, s>>>(a);
+    }
   } else if (!inv) {
     smem_opt_in(k4_fwd_y<T, NB>, of);
     k4_fwd_y<T, NB><<<g, 256, smem, s>>>(a);
@@ -63,7 +79,7 @@ static void launch_z4(const MvArgs<T>& a, dim3 g, size_t smem, cudaStream_t s) {
     k4_zp<NB, PWL, OP><<<g, kZpThreads, smem, s>>>(a);
   } else if constexpr (std::is_same<T, ff>::value) {
     smem_opt_in(k4_zf<NB, PWL, OP>, o);
-    k4_zf<NB, PWL, OP><<<g, 256, smem, s>>>(a);
+    k4_zf<NB, PWL, OP><<<g, kZfThreads, smem, s>>>(a);
   } else {
     smem_opt_in(k4_z<T, NB, PWL, OP>, o);
     k4_z<T, NB, PWL, OP><<<g, 256, smem, s>>>(a);

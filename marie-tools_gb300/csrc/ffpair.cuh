@@ -67,25 +67,36 @@ __device__ __forceinline__ ffc2 mul_w(ffc2 b) {
   return {f2_swap(b.hi) * sg, f2_swap(b.lo) * sg};
 }
 
-// a times the per-lane float-float constant k, given k.hi and the negated
-// -k.hi, -k.lo
-__device__ __forceinline__ ffc2 mulk(ffc2 a, f2 khi, f2 nkhi, f2 nklo) {
-  const f2 p = a.hi * khi;
-  f2 e = fma2(a.hi, nkhi, p);   // p - a.hi*k.hi (exact)
-  e = fma2(a.hi, nklo, e);
-  e = fma2(a.lo, nkhi, e);
+// Lanes (d0, d1) of two double constants: the high part and the negated high,
+// low and third part.  The third (one FMA) keeps a constant's representation error,
+// the same in every transform of a product, from adding up over the six.
+struct kff {
+  f2 hi, nhi, nlo, n3;
+};
+__device__ __forceinline__ kff kff_make(double d0, double d1) {
+  const ff a(d0), b(d1);
+  return {f2_make(a.hi, b.hi), f2_make(-a.hi, -b.hi), f2_make(-a.lo, -b.lo),
+          f2_make((float)((double)a.hi - d0 + (double)a.lo), (float)((double)b.hi - d1 + (double)b.lo))};
+}
+
+// a times the per-lane constant k
+__device__ __forceinline__ ffc2 mulk(ffc2 a, const kff& k) {
+  const f2 p = a.hi * k.hi;
+  f2 e = fma2(a.hi, k.nhi, p);   // p - a.hi*k.hi (exact)
+  e = fma2(a.hi, k.nlo, e);
+  e = fma2(a.lo, k.nhi, e);
+  e = fma2(a.hi, k.n3, e);
   const f2 h = p - e;
   return {h, (p - h) - e};
 }
 
-// Lanes (d0, d1) of two double constants as float-float: hi and the negated
-// hi, lo.
-struct kff {
-  f2 hi, nhi, nlo;
-};
-__device__ __forceinline__ kff kff_make(double d0, double d1) {
-  const ff a(d0), b(d1);
-  return {f2_make(a.hi, b.hi), f2_make(-a.hi, -b.hi), f2_make(-a.lo, -b.lo)};
+// (p - e) + (q - g), p and q products with the errors e and g, normalised once
+__device__ __forceinline__ ffc2 sum2(f2 p, f2 e, f2 q, f2 g) {
+  const f2 s = p + q;
+  const f2 bb = s - p;
+  const f2 l = ((p - (s - bb)) + (q - bb)) - (e + g);
+  const f2 h = s + l;
+  return {h, l - (h - s)};
 }
 
 // v * exp(-+ i theta) for cos(theta) = c, sin(theta) = s (forward: minus):
@@ -95,9 +106,12 @@ __device__ __forceinline__ ffc2 rotf(ffc2 v, double c, double s) {
   const double ws = INV ? s : -s;
   if (c == 0.0) return ws > 0 ? mul_w<true>(v) : mul_w<false>(v);
   const kff C = kff_make(c, c), B = kff_make(-ws, ws);
-  const ffc2 a = mulk(v, C.hi, C.nhi, C.nlo);
-  const ffc2 b = mulk(ffc2_swap(v), B.hi, B.nhi, B.nlo);
-  return a + b;
+  const ffc2 w = ffc2_swap(v);
+  const f2 p = v.hi * C.hi, q = w.hi * B.hi;
+  f2 e = fma2(v.hi, C.nhi, p), g = fma2(w.hi, B.nhi, q);
+  e = fma2(v.hi, C.n3, fma2(v.lo, C.nhi, fma2(v.hi, C.nlo, e)));
+  g = fma2(w.hi, B.n3, fma2(w.lo, B.nhi, fma2(w.hi, B.nlo, g)));
+  return sum2(p, e, q, g);
 }
 
 // Twiddle table entry for w = wr + i wi: hi = ((wr.hi, wr.hi), (-wi.hi,
@@ -108,18 +122,9 @@ struct __align__(16) fftw {
 __device__ __forceinline__ fftw fftw_make(cplx<ff> w) {
   return {f2_make(w.x.hi, w.x.hi), f2_make(-w.y.hi, w.y.hi), f2_make(w.x.lo, w.x.lo), f2_make(-w.y.lo, w.y.lo)};
 }
-// v * w (CONJ: v * conj(w))
-template <bool CONJ>
-__device__ __forceinline__ ffc2 tw_mulf(ffc2 v, const fftw& t) {
-  const f2 zero = f2_make(0.f, 0.f);
-  const ffc2 a = mulk(v, t.rh, zero - t.rh, zero - t.rl);
-  const ffc2 vs = ffc2_swap(v);
-  const ffc2 b = CONJ ? mulk(vs, zero - t.ih, t.ih, t.il) : mulk(vs, t.ih, zero - t.ih, zero - t.il);
-  return a + b;
-}
 
 // ---------------------------------------------------------------------------
-// DFTs of lengths 1-8 and 16, in place, natural order, no scaling.
+// DFTs of lengths 1-8, in place, natural order, no scaling.
 // ---------------------------------------------------------------------------
 
 template <bool INV>
@@ -183,8 +188,8 @@ __device__ __forceinline__ void dftf_prime(ffc2* v) {
       const double c = PrimeTab<R>::c(mm);
       const double sn = m <= H ? PrimeTab<R>::s(mm) : -PrimeTab<R>::s(mm);
       const kff C = kff_make(c, c), S = kff_make(sn, sn);
-      re = re + mulk(s[j - 1], C.hi, C.nhi, C.nlo);
-      const ffc2 t = mulk(d[j - 1], S.hi, S.nhi, S.nlo);
+      re = re + mulk(s[j - 1], C);
+      const ffc2 t = mulk(d[j - 1], S);
       im = j == 1 ? t : im + t;
     }
     const ffc2 wim = mul_w<INV>(im);
@@ -213,25 +218,6 @@ __device__ __forceinline__ void dftf6(ffc2* v) {
   }
 }
 
-template <bool INV>
-__device__ __forceinline__ void dftf16(ffc2* v) {
-  ffc2 A[16];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    ffc2 t[4] = {v[b], v[4 + b], v[8 + b], v[12 + b]};
-    dftf4<INV>(t);
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) A[b * 4 + k1] = (b * k1 == 0) ? t[k1] : rotf<INV>(t[k1], c16(b * k1), s16(b * k1));
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) {
-    ffc2 t[4] = {A[k1], A[4 + k1], A[8 + k1], A[12 + k1]};
-    dftf4<INV>(t);
-#pragma unroll
-    for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = t[k2];
-  }
-}
-
 template <bool INV, int N>
 __device__ __forceinline__ void dftf(ffc2* v) {
   if constexpr (N == 1) {
@@ -243,21 +229,9 @@ __device__ __forceinline__ void dftf(ffc2* v) {
     dftf6<INV>(v);
   } else if constexpr (N == 8) {
     dftf8<INV>(v);
-  } else if constexpr (N == 16) {
-    dftf16<INV>(v);
   } else {
     dftf_prime<INV, N>(v);
   }
-}
-
-template <bool INV, int N>
-__device__ __forceinline__ void dftn_ffc2(cplx<ff>* v) {
-  ffc2 u[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) u[i] = to_ffc2(v[i]);
-  dftf<INV, N>(u);
-#pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = from_ffc2(u[i]);
 }
 
 }  // namespace marie

@@ -59,7 +59,7 @@ struct PrecState {
   cplx<T>* chi = nullptr;     // Ns
   cplx<T>* GN = nullptr;      // nblkN * oct
   cplx<T>* GK = nullptr;      // nblkK * oct
-  cplx<T>* GNf = nullptr;     // octant columns [ky <= n2][kx <= n1], each [kz][blk] (four-step grids; complex64: pair layout)
+  cplx<T>* GNf = nullptr;     // octant columns [ky <= n2][kx <= n1], each [kz][blk] (four-step grids; complex64: pair layout, float-float: [blk][kz & 1][kz/2])
   cplx<T>* GKf = nullptr;     // the same for K (complex64)
   cplx<T>* T1 = nullptr;      // ws_rhs * C * n3 * n2 * 2n1
   cplx<T>* S = nullptr;       // ws_rhs * C * 2n2 * n3 * 2n1

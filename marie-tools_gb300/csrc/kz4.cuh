@@ -27,10 +27,6 @@ __device__ __forceinline__ int zpos(int j, int k1) { return j * 16 + (k1 ^ j); }
 __device__ __forceinline__ cplx<double> shfl_xor_c(cplx<double> v, int m) {
   return {__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m)};
 }
-__device__ __forceinline__ cplx<ff> shfl_xor_c(cplx<ff> v, int m) {
-  return {ff(__shfl_xor_sync(0xffffffffu, v.x.hi, m), __shfl_xor_sync(0xffffffffu, v.x.lo, m)),
-          ff(__shfl_xor_sync(0xffffffffu, v.y.hi, m), __shfl_xor_sync(0xffffffffu, v.y.lo, m))};
-}
 
 // One entry of the single-point Green multiply (entries sorted by block;
 // every index a compile-time constant).  gp points at the point's U block

@@ -10,9 +10,9 @@
 // makes one shared-memory round trip (the z pass four: forward, multiply,
 // inverse), and every index is a shift or a multiply by a constant.
 // Spectra are kept in natural frequency order: position k of half alpha holds
-// frequency 2k + alpha.  The x and y passes here serve complex128; complex64 has
-// its own (xy4c.cuh).  Layouts in HBM are those of matvec.cuh over the caller's
-// rows y < g2 and slices z < g3.
+// frequency 2k + alpha.  The x and y passes here serve native complex128;
+// complex64 and float-float have their own (xy4c.cuh, xy4f.cuh).  Layouts in HBM
+// are those of matvec.cuh over the caller's rows y < g2 and slices z < g3.
 #pragma once
 
 #include "matvec.cuh"
@@ -79,15 +79,9 @@ __device__ __forceinline__ void dft6(cplx<T>* v) {
   }
 }
 
-// Float-float DFTs run in packed (re, im) pairs (ffpair.cuh).
-template <bool INV, int N>
-__device__ __forceinline__ void dftn_ffc2(cplx<ff>* v);
-
 template <typename T, bool INV, int N>
 __device__ __forceinline__ void dftn(cplx<T>* v) {
-  if constexpr (std::is_same<T, ff>::value && N > 1) {
-    dftn_ffc2<INV, N>(v);
-  } else if constexpr (N == 1) {
+  if constexpr (N == 1) {
   } else if constexpr (N == 6) {
     dft6<T, INV>(v);
   } else if constexpr (N == 16) {
@@ -364,4 +358,5 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_y(MvArgs<T
 #include "kz4.cuh"
 #include "xy4c.cuh"
 #include "kz4p.cuh"
+#include "xy4f.cuh"
 #include "kz4f.cuh"

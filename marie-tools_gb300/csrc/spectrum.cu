@@ -125,7 +125,9 @@ __global__ void k_oct_store(const zd* tmp, cplx<T>* dst, int nkx, int nky, int n
 // Spectrum of one block for the four-step z pass, octant columns: for the
 // columns kx in [0, n1], ky in [0, n2] all 2n3 frequencies kz, the z mirror
 // sign applied; the mirrored columns follow by signs of the components
-// (mirror_mask).  dst[((ky*(n1+1) + kx)*2n3 + kz)*U + blk].
+// (mirror_mask).  dst[((ky*(n1+1) + kx)*2n3 + kz)*U + blk]; float-float
+// ((ky*(n1+1) + kx)*U + blk)*2n3 + (kz & 1)*n3 + kz/2: threads of neighbouring
+// frequencies read neighbouring values.
 template <typename T>
 __global__ void k_full_store(const zd* tmp, cplx<T>* dst, int n1, int n2, int n3, int U, int blk, int s3, double scl) {
   const int m3 = 2 * n3;
@@ -140,7 +142,8 @@ __global__ void k_full_store(const zd* tmp, cplx<T>* dst, int n1, int n2, int n3
     const bool mz = kz > n3;
     const double sg = (double)(mz ? s3 : 1) * scl;
     const zd v = tmp[kx + (int64_t)nkx * (ky + (int64_t)nky * (mz ? m3 - kz : kz))];
-    dst[idx * U + blk] = cplx<T>{(T)(v.x * sg), (T)(v.y * sg)};
+    const int64_t o = std::is_same<T, ff>::value ? (r * U + blk) * m3 + (kz & 1) * n3 + (kz >> 1) : idx * U + blk;
+    dst[o] = cplx<T>{(T)(v.x * sg), (T)(v.y * sg)};
   }
 }
 
