@@ -350,13 +350,85 @@ __device__ __forceinline__ void zitem(cplx<T>* buf, int o0, int o1, int qstride,
   }
 }
 
+// One output group P (four moments) of the PWL product at one point, P a value of
+// the thread: the table of one (P, Q) block of four by four serves every group.
+// The blocks are the octant value's, so v's components carry the mirrors' signs.
+// N: block (j, k = PQ_N(P, Q) - 1) at 6j + k; K: (j, k = 3 - P - Q) at 3j + k, with
+// the sign of (0, 1) for Q = P + 1 and the other for Q = P + 2 (mod 3).
+struct PwlBlock {
+  int jl[4][4];          // Tucker index j of entry (l, lp)
+  int sg[4][4];          // its sign (K: for Q = P + 1)
+};
+template <int OP>
+constexpr PwlBlock make_pwl_block() {
+  using Tab = OpTab<true, OP>;
+  constexpr int q0 = OP >= 2 ? 4 : 0;
+  PwlBlock t{};
+  for (int i = 0; i < Tab::NE; ++i) {
+    const OpEntry e = Tab::L.e[i];
+    if (e.p < 4 && e.q >= q0 && e.q < q0 + 4) {
+      t.jl[e.p][e.q - q0] = e.blk / (OP >= 2 ? 3 : 6);
+      t.sg[e.p][e.q - q0] = e.sgn;
+    }
+  }
+  return t;
+}
+template <int OP, bool NEG>
+__device__ __forceinline__ void zgroup_block(cplx<double>* y, const cplx<double>* x, const cplx<double>* gp,
+                                             int64_t gblk) {
+  constexpr PwlBlock TB = make_pwl_block<OP>();
+  constexpr int nk = OP >= 2 ? 3 : 6;
+#pragma unroll
+  for (int j = 0; j < 10; ++j) {
+    cplx<double> g = ldg_c(gp + nk * j * gblk);
+    if constexpr ((OP & 1) != 0) g = conjg(g);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+#pragma unroll
+      for (int lp = 0; lp < 4; ++lp) {
+        if (TB.jl[l][lp] == j) {
+          if ((TB.sg[l][lp] > 0) != NEG) fma_c(y[l], g, x[lp]);
+          else fms_c(y[l], g, x[lp]);
+        }
+      }
+    }
+  }
+}
+template <int OP>
+__device__ __forceinline__ void zgroup(cplx<double>* y, const cplx<double>* v, int qstride, unsigned flips, unsigned oflips,
+                                       const cplx<double>* gp, int64_t gblk, int P) {
+#pragma unroll
+  for (int l = 0; l < 4; ++l) y[l] = cplx<double>{0, 0};
+  auto load = [&](cplx<double>* x, int Q) {
+#pragma unroll
+    for (int lp = 0; lp < 4; ++lp)
+      x[lp] = flip_c(v[(4 * Q + lp) * qstride], (flips >> (4 * Q + lp)) << 31);
+  };
+  cplx<double> x[4];
+  if constexpr (OP >= 2) {
+    const int Q1 = P == 2 ? 0 : P + 1, Q2 = 3 - P - Q1;
+    load(x, Q1);
+    zgroup_block<OP, false>(y, x, gp + Q2 * gblk, gblk);   // k = 3 - P - Q
+    load(x, Q2);
+    zgroup_block<OP, true>(y, x, gp + Q1 * gblk, gblk);
+  } else {
+#pragma unroll 1
+    for (int Q = 0; Q < 3; ++Q) {
+      load(x, Q);
+      zgroup_block<OP, false>(y, x, gp + (P + Q + (P > 0 && Q > 0 ? 1 : 0)) * gblk, gblk);
+    }
+  }
+#pragma unroll
+  for (int l = 0; l < 4; ++l) y[l] = flip_c(y[l], (oflips >> (4 * P + l)) << 31);
+}
+
 // ---------------------------------------------------------------------------
 // Pass Z (fused).  grid (ceil(2n1/TX), 2n2, nbundle)
 // sequences s = ((gamma*C + c)*TX + t)*R + r, length n3; row i of buf holds
 // the z-sample (on load) / frequency (after the DIT) i of every sequence.
 // ---------------------------------------------------------------------------
 template <typename T, bool PWL, int OP>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_z(MvArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) k_z(MvArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int b = blockIdx.z;
   if (!bundle_active(a, b)) return;
@@ -398,7 +470,34 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) k_z(MvArgs<T> a) 
   const int kyo = my ? 2 * n2 - ky : ky;
   const int nko = n3 + 1;
   const int64_t gblk = (int64_t)(n2 + 1) * (n1 + 1) * nko;
-  for (int i = threadIdx.x; i < n3 * W; i += blockDim.x) {
+  if constexpr (PWL && sizeof(T) == 8) {
+    // FP64 (two FMAs per clock and SM): three threads per frequency, each one
+    // output group, so that every scheduler has the same number of warps to serve
+    // (with an item above per thread 160 on 256 threads at n3 = 40: 48 x 56 x 40
+    // 3.69 ms a product, here 2.60).  The outputs go back when all have read.
+    const int per = blockDim.x / 3, P = threadIdx.x / per, total = 2 * n3 * W;
+    for (int i0 = 0; i0 < total; i0 += per) {
+      const int i = i0 + threadIdx.x - P * per;
+      const int e = i % W, kz = i / W;
+      const int t = e / R;
+      const bool act = P < 3 && i < total && t < tx;
+      const int kxp = k0 + t;
+      const int alpha = kxp / n1, px = kxp - alpha * n1;
+      const int kx = act ? 2 * a.ax.kofp[px] + alpha : 0;
+      const bool mx = kx > n1, mz = kz > n3;
+      const int kxo = mx ? 2 * n1 - kx : kx, kzo = mz ? 2 * n3 - kz : kz;
+      const unsigned flips = mirror_flips<true>(mx, my) ^ (mz ? mirror_mask<true>(2) : 0u);
+      const unsigned oflips = OP >= 2 && (mx ^ my ^ mz) ? ~flips : flips;   // K: one more sign per mirror
+      cplx<T>* v = buf + (kz >> 1) * es + (kz & 1) * C * W + e;
+      cplx<T> y[4];
+      if (act) zgroup<OP>(y, v, W, flips, oflips, a.G + ((int64_t)kyo * (n1 + 1) + kxo) * nko + kzo, gblk, P);
+      __syncthreads();
+      if (act) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l) v[(4 * P + l) * W] = y[l];
+      }
+    }
+  } else for (int i = threadIdx.x; i < n3 * W; i += blockDim.x) {
     const int e = i % W, u = i / W;
     const int t = e / R;
     if (t >= tx) continue;
