@@ -303,19 +303,60 @@ struct CallTiles {
   int R, TY, TXY, TX, TZY;
 };
 
-static int pow2floor(int v) {
-  int p = 1;
-  while (p * 2 <= v) p *= 2;
-  return p;
+// Bundle size R of nr right-hand sides: a power of two, <= the z tile width Wz.  The
+// last bundle computes its empty places too, so few of them come first; a wide
+// bundle shares each Green value and twiddle, worth a quarter of a product between
+// one and many in complex64, a sixteenth in the arithmetic-bound precisions (per
+// right-hand side at R = 1 / 2 / 4: 96^3 PWL complex64 880 / 818 / 796 us, 112^3 PWC
+// 303 / 274 / 253, 48^3 PWL 150 / 137 / 116, float-float 557 / 552 / 540).  Against
+// the largest R <= nr: 96^3 PWL five 6.37 -> 4.41 ms, three 3.27 -> 2.68; complex128
+// 33 x 30 x 28 PWL three 3.38 -> 2.68; seven stay at R = 4 in complex64 (112^3 PWC
+// 2.03 ms, 2.10 at R = 1).
+template <typename T>
+static int bundle_size(int nr, int Wz, double* least = nullptr) {
+  const double share = sizeof(T) == 4 ? 0.25 : 0.0625;
+  int best = 1;
+  double lc = 0;
+  for (int R = 1; R <= Wz && R <= std::max(1, nr); R *= 2) {
+    const double cost = (double)((nr + R - 1) / R * R) * (1 + share / R);
+    if (R == 1 || cost <= lc) {
+      best = R;
+      lc = cost;
+    }
+  }
+  if (least) *least = lc;
+  return best;
 }
 
-// Bundle size R (a power of two, <= the z tile width) and the tiles of one
-// chunk of nr right-hand sides.  fast: four-step passes (wider x/y tiles).
+// Right-hand sides of the next chunk out of nr that fit the workspace (complex64):
+// where one product fills the chip for several waves (grid values kSplitElements),
+// the powers of two of a count go by themselves if that saves a twentieth of the
+// bundles' cost.  In chunks against whole: 96^3 PWL three 2.61 / 2.67 ms, five 4.12 /
+// 4.40, seven 5.80 / 6.42; 112^3 PWC seven 1.96 / 2.02; 60 x 77 x 90 PWL three 1.53 /
+// 1.55; but 64^3 PWL (3.1 million values) three 0.85 / 0.83, 48^3 PWL seven 0.96 / 0.93.
+constexpr int64_t kSplitElements = 1 << 22;
+static double split_cost(int nr, int Wz, int* first) {
+  double whole;
+  bundle_size<float>(nr, Wz, &whole);
+  *first = nr;
+  int q = 1, rest;
+  while (q * 2 <= nr) q *= 2;
+  if (q == nr || q > Wz) return whole;
+  double head;
+  bundle_size<float>(q, Wz, &head);
+  const double parts = head + split_cost(nr - q, Wz, &rest);
+  if (parts > 0.95 * whole) return whole;
+  *first = q;
+  return parts;
+}
+
+// Bundle size R and the tiles of one chunk of nr right-hand sides.  fast: four-step
+// passes (wider x/y tiles).
 template <typename T>
 static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, bool fast) {
   CallTiles t;
   const int Wz = ps.TX;
-  t.R = pow2floor(std::max(1, std::min(Wz, nr)));
+  t.R = bundle_size<T>(nr, Wz);
   const int n1 = ps.m1, n2 = ps.m2;
   const int wxy = (sizeof(T) == 4 ? 16 : 8) * (fast ? 2 : 1);   // row-tile width of the x/y passes
   t.TY = std::max(1, std::min(n2, wxy / t.R));
@@ -484,10 +525,11 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
     if (h->tkf.active && (op == OP_N || op == OP_N_ADJ) && !env_int("MARIE_GENERIC_FFT", 0))
       MARIE_TRY(tucker_expand_c64(h, stream));
   }
-  for (int r0 = 0; r0 < nrhs; r0 += ps.ws_rhs) {
-    const int nr = std::min(ps.ws_rhs, nrhs - r0);
-    // a padded state has the four-step passes only
-    const bool fast = four_step_op(h, ps, op) && (ps.padded || !env_int("MARIE_GENERIC_FFT", 0));
+  // a padded state has the four-step passes only
+  const bool fast = four_step_op(h, ps, op) && (ps.padded || !env_int("MARIE_GENERIC_FFT", 0));
+  for (int r0 = 0, nr; r0 < nrhs; r0 += nr) {
+    nr = std::min(ps.ws_rhs, nrhs - r0);
+    if (fast && sizeof(T) == 4 && (int64_t)C * n1 * n2 * n3 >= kSplitElements) split_cost(nr, ps.TX, &nr);
     const CallTiles ct = call_tiles(h, ps, nr, fast);
     const int nb = (nr + ct.R - 1) / ct.R;
     a.R = ct.R;
