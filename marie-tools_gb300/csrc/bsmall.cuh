@@ -8,21 +8,45 @@
 // a GEMM's 128-wide tiles of a p-wide result are far from: 48^3 PWL, eight
 // right-hand sides, the emulated GEMMs took 0.8 ms for a step's projection and
 // update and 1.3 ms for its block QR, two and a half times the operator's 0.95
-// ms (the whole solve 947 -> 463 ms).
+// ms (the whole solve 947 -> 463 ms).  At 240 vectors of 396960 the two take 219 and
+// 228 us (HBM alone 116, the FP32 work alone 82): many loads in flight beside the
+// arithmetic are what counts, so few registers a thread, and sums over a warp that
+// exchange each value once (k_tall_cn with four columns a pass and a butterfly per
+// value 266 us; k_tall_comb with half the loads in flight and CTAs of 256 414 us).
 #pragma once
 
 namespace marie {
 
 constexpr int kTallMax = 16;          // largest p of these kernels
 constexpr int kTallThreads = 256;
-constexpr int kTallCtas = 2 * 152;    // row ranges (partial sums per entry)
+constexpr int kTallCtas = 3 * 152;    // most row ranges (partial sums per entry)
+constexpr int kCombThreads = 128;
 
 // Rows of B staged in shared memory per piece and columns of A per warp pass.
 template <int P>
 struct Tall {
   static constexpr int rows = 4096 / P;
-  static constexpr int cols = P <= 8 ? 4 : 2;
+  static constexpr int cols = P <= 4 ? 4 : 2;
+  static constexpr int ctas = P <= 8 ? 3 : 2;   // per SM, of k_tall_cn
 };
+
+// The V (a multiple of 32) values of every lane summed over the warp: value
+// lane*V/32 + i ends in a[i] of its lane.  Each step halves the values a lane
+// keeps: V - V/32 exchanges, where a butterfly per value takes 5*V.
+template <int V>
+__device__ __forceinline__ void warp_transpose_sum(float* a, int lane) {
+#pragma unroll
+  for (int o = 16, h = V / 2; o > 0; o >>= 1, h >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < V / 2; ++i) {
+      if (i < h) {
+        const float keep = up ? a[i + h] : a[i], send = up ? a[i] : a[i + h];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+  }
+}
 
 // Partial products of the CTA's rows: part[(c*M + m)*gridDim.x + blockIdx.x].
 // The CTA stages `rows` rows of B, its warps take groups of `cols` columns of A
@@ -31,11 +55,11 @@ struct Tall {
 // accumulators in shared memory.  flag (may be null): set to 2 if a value of B
 // is not finite.
 template <int P>
-__global__ void __launch_bounds__(kTallThreads) k_tall_cn(const cplx<float>* __restrict__ A,
+__global__ void __launch_bounds__(kTallThreads, Tall<P>::ctas) k_tall_cn(const cplx<float>* __restrict__ A,
                                                           const cplx<float>* __restrict__ B, int64_t Nb, int M, int p,
                                                           cplx<float>* __restrict__ part, int* flag) {
   extern __shared__ __align__(16) unsigned char tall_smem[];
-  constexpr int RC = Tall<P>::rows, CW = Tall<P>::cols, kWarps = kTallThreads / 32;
+  constexpr int RC = Tall<P>::rows, CW = Tall<P>::cols, V = 2 * CW * P, kWarps = kTallThreads / 32;
   float2* bt = reinterpret_cast<float2*>(tall_smem);        // [P][RC]
   const int ngroups = (M + CW - 1) / CW;
   int split = 1;
@@ -66,12 +90,10 @@ __global__ void __launch_bounds__(kTallThreads) k_tall_cn(const cplx<float>* __r
       const float2* a[CW];
 #pragma unroll
       for (int k = 0; k < CW; ++k) a[k] = A2 + (int64_t)min(g * CW + k, M - 1) * Nb + base;
-      float2 s[CW][P];
+      float s[V];
 #pragma unroll
-      for (int k = 0; k < CW; ++k)
-#pragma unroll
-        for (int c = 0; c < P; ++c) s[k][c] = make_float2(0.f, 0.f);
-#pragma unroll 2
+      for (int i = 0; i < V; ++i) s[i] = 0.f;
+#pragma unroll 4
       for (int st = s0; st < s1; ++st) {
         const int r = st * 32 + lane;
         float2 v[CW];
@@ -82,27 +104,19 @@ __global__ void __launch_bounds__(kTallThreads) k_tall_cn(const cplx<float>* __r
           const float2 w = bt[c * RC + (r < RC ? r : RC - 1)];
 #pragma unroll
           for (int k = 0; k < CW; ++k) {
-            s[k][c].x = fmaf(v[k].x, w.x, fmaf(v[k].y, w.y, s[k][c].x));
-            s[k][c].y = fmaf(v[k].x, w.y, fmaf(-v[k].y, w.x, s[k][c].y));
+            float* q = s + 2 * (k * P + c);
+            q[0] = fmaf(v[k].x, w.x, fmaf(v[k].y, w.y, q[0]));
+            q[1] = fmaf(v[k].x, w.y, fmaf(-v[k].y, w.x, q[1]));
           }
         }
       }
+      warp_transpose_sum<V>(s, lane);
 #pragma unroll
-      for (int k = 0; k < CW; ++k)
-#pragma unroll
-        for (int c = 0; c < P; ++c) {
-          float2 t = s[k][c];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-            t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
-          }
-          if (lane == 0 && g * CW + k < M && c < p) {
-            float2& q = acc[(int64_t)sp * M * p + c * M + g * CW + k];
-            q.x += t.x;
-            q.y += t.y;
-          }
-        }
+      for (int i = 0; i < V / 32; ++i) {
+        const int id = lane * (V / 32) + i, k = id / (2 * P), c = (id >> 1) % P;
+        if (g * CW + k < M && c < p)
+          reinterpret_cast<float*>(acc)[2 * ((int64_t)sp * M * p + c * M + g * CW + k) + (id & 1)] += s[i];
+      }
     }
   }
   if (__syncthreads_or(bad) && flag && threadIdx.x == 0) *(volatile int*)flag = 2;
@@ -138,20 +152,20 @@ __global__ void k_tall_sum(const cplx<float>* __restrict__ part, int nparts, int
 // C_c[i] = alpha * sum_m A_m[i] X[m + M*c] + beta * C_c[i], two rows per thread
 // (each coefficient read from shared memory serves both); beta 0 or 1.
 template <int P>
-__global__ void __launch_bounds__(kTallThreads) k_tall_comb(const cplx<float>* __restrict__ A,
+__global__ void __launch_bounds__(kCombThreads) k_tall_comb(const cplx<float>* __restrict__ A,
                                                             const cplx<float>* __restrict__ X, int64_t Nb, int M,
                                                             int p, float alpha, float beta, cplx<float>* C) {
   extern __shared__ __align__(16) unsigned char tall_smem[];
   float2* x = reinterpret_cast<float2*>(tall_smem);         // [M][P]
-  for (int i = threadIdx.x; i < M * P; i += kTallThreads) {
+  for (int i = threadIdx.x; i < M * P; i += kCombThreads) {
     const int m = i / P, c = i - m * P;
     const cplx<float> v = c < p ? X[m + (int64_t)M * c] : cplx<float>{0.f, 0.f};
     x[i] = make_float2(alpha * v.x, alpha * v.y);
   }
   __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * kTallThreads * 2;
-  for (int64_t i0 = (int64_t)blockIdx.x * kTallThreads * 2 + threadIdx.x; i0 < Nb; i0 += stride) {
-    const int64_t i1 = i0 + kTallThreads;
+  const int64_t stride = (int64_t)gridDim.x * kCombThreads * 2;
+  for (int64_t i0 = (int64_t)blockIdx.x * kCombThreads * 2 + threadIdx.x; i0 < Nb; i0 += stride) {
+    const int64_t i1 = i0 + kCombThreads;
     const bool two = i1 < Nb;
     float2 s[2][P];
 #pragma unroll
@@ -166,7 +180,7 @@ __global__ void __launch_bounds__(kTallThreads) k_tall_comb(const cplx<float>* _
         }
       }
     }
-#pragma unroll 4
+#pragma unroll 8
     for (int m = 0; m < M; ++m) {
       const cplx<float> u = A[(int64_t)m * Nb + i0];
       const cplx<float> t = two ? A[(int64_t)m * Nb + i1] : cplx<float>{0.f, 0.f};
@@ -199,7 +213,7 @@ static marie_status tall_cn(int64_t Nb, int M, int p, const cplx<float>* A, cons
                             cplx<float>* part, int* flag, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
   smem_opt_in_device((const void*)k_tall_cn<P>, done);
-  const int ctas = (int)std::min<int64_t>(kTallCtas, (Nb + 255) / 256);
+  const int ctas = (int)std::min<int64_t>(Tall<P>::ctas * 152, (Nb + 255) / 256);
   k_tall_cn<P><<<ctas, kTallThreads, tall_cn_smem<P>(M, p), s>>>(A, B, Nb, M, p, part, flag);
   MARIE_LAUNCH_CHECK();
   k_tall_sum<<<(M * p + 7) / 8, 256, 0, s>>>(part, ctas, M * p, H);
@@ -211,9 +225,9 @@ static marie_status tall_comb(int64_t Nb, int M, int p, float alpha, const cplx<
                               float beta, cplx<float>* C, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
   smem_opt_in_device((const void*)k_tall_comb<P>, done);
-  const int64_t need = (Nb + 2 * kTallThreads - 1) / (2 * kTallThreads);
-  k_tall_comb<P><<<(unsigned)std::min<int64_t>(need, 8 * 152), kTallThreads, tall_comb_smem<P>(M), s>>>(A, X, Nb, M, p,
-                                                                                                      alpha, beta, C);
+  const int64_t need = (Nb + 2 * kCombThreads - 1) / (2 * kCombThreads);
+  k_tall_comb<P><<<(unsigned)std::min<int64_t>(need, 16 * 152), kCombThreads, tall_comb_smem<P>(M), s>>>(
+      A, X, Nb, M, p, alpha, beta, C);
   MARIE_LAUNCH_CHECK();
   return MARIE_OK;
 }
