@@ -699,7 +699,7 @@ static marie_status validate_desc(const marie_vie_desc* d, std::vector<int64_t>&
 // 2n - 1 with zeros at the offsets n..m-1 gives the same on the grid, embed.h;
 // rows, slices and columns beyond the grid are never stored or read).  The
 // generic passes take four to five times as long per grid point (60 x 77 x 90
-// PWL, three right-hand sides: 6.5 ms against 1.9; 24^3 PWL one: 91 against 81
+// PWL, three right-hand sides: 6.5 ms against 1.5; 24^3 PWL one: 91 against 81
 // us at 2.4 times the volume; 17 x 40 x 40 PWL four: 491 against 339 at 2.7), so
 // padding pays up to about three times the volume.  Not under a memory cap, nor
 // where the larger work arrays and spectra would not fit easily: the generic

@@ -294,7 +294,7 @@ static marie_status proj_cn(marie_vie* h, BlockWork& w, cublasHandle_t bl, int64
       MARIE_CUDA_TRY(cudaHostGetDevicePointer((void**)&qd, h->bio, 0));
       flag = (int*)(qd + bio_err(w.p, w.mb));
     }
-    return tall_cn(w.Nb, (int)m, w.p, A, B, H, w.part, flag, s);
+    return tall_cn(w.Nb, (int)m, w.p, A, B, H, w.part, w.part_cap, flag, s);
   }
   if (w.tc) {
     unsigned char* qd = nullptr;
@@ -351,7 +351,7 @@ static marie_status block_qr(marie_vie* h, BlockWork& w, cublasHandle_t bl, cplx
     // the Gram matrix in cuBLAS's FP32-accurate products: the Cholesky
     // factor needs its small eigenvalues (the tensor-core kernel's ~1e-6
     // relative error is enough for the projections, not here)
-    if (w.tall) MARIE_TRY(tall_cn(Nb, p, p, a, a, w.Gm, w.part, nullptr, s));
+    if (w.tall) MARIE_TRY(tall_cn(Nb, p, p, a, a, w.Gm, w.part, w.part_cap, nullptr, s));
     else MARIE_TRY(cgemm_cn(bl, p, p, Nb, a, Nb, a, Nb, w.Gm, p, w.part, w.part_cap, s));
     MARIE_TRY(bio_move(h, bio_gm(p, w.mb), w.Gm, (size_t)p * p * 8, true, s));
     MARIE_CUDA_TRY(cudaStreamSynchronize(s));
@@ -418,9 +418,11 @@ static marie_status block_work_alloc(marie_vie* h, BlockWork& w, int pmax, int m
   MARIE_TRY(sc.get(&w.Gm, (size_t)pmax * pmax));
   MARIE_TRY(sc.get(&w.Sm, (size_t)(mb + 1) * pmax * pmax));
   MARIE_TRY(sc.get(&w.map, (size_t)pmax + 1));
-  // a refinement step may solve fewer columns than pmax and take bsmall.cuh then
+  // a refinement step may solve fewer columns than pmax and take bsmall.cuh then,
+  // on fewer CTAs where a memory cap leaves no room for every CTA's sums
   const int64_t ps = std::min(pmax, kTallMax);
-  w.part_cap = std::max((int64_t)65 * mb * pmax * pmax, (int64_t)kTallCtas * mb * ps * ps);
+  w.part_cap = (int64_t)65 * mb * pmax * pmax;
+  if (h->mem_cap == 0) w.part_cap = std::max(w.part_cap, (int64_t)kTallCtas * mb * ps * ps);
   MARIE_TRY(sc.get(&w.part, (size_t)w.part_cap));
   w.tpart_floats = block_gemm_part_floats(Nb, mb * std::min(pmax, 64));
   if (pmax <= 64 && Nb % 2 == 0 && proj_tcgen05()) MARIE_TRY(sc.get(&w.tpart, (size_t)w.tpart_floats));

@@ -210,10 +210,11 @@ inline size_t tall_comb_smem(int M) { return (size_t)M * P * 8; }
 
 template <int P>
 static marie_status tall_cn(int64_t Nb, int M, int p, const cplx<float>* A, const cplx<float>* B, cplx<float>* H,
-                            cplx<float>* part, int* flag, cudaStream_t s) {
+                            cplx<float>* part, int64_t part_cap, int* flag, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
   smem_opt_in_device((const void*)k_tall_cn<P>, done);
-  const int ctas = (int)std::min<int64_t>(Tall<P>::ctas * 152, (Nb + 255) / 256);
+  const int64_t rows = std::min<int64_t>(Tall<P>::ctas * 152, (Nb + 255) / 256);
+  const int ctas = (int)std::min<int64_t>(rows, part_cap / ((int64_t)M * p));
   k_tall_cn<P><<<ctas, kTallThreads, tall_cn_smem<P>(M, p), s>>>(A, B, Nb, M, p, part, flag);
   MARIE_LAUNCH_CHECK();
   k_tall_sum<<<(M * p + 7) / 8, 256, 0, s>>>(part, ctas, M * p, H);
@@ -237,10 +238,10 @@ static bool tall_fits(int64_t M, int p) {
          tall_comb_smem<16>((int)std::min<int64_t>(M, 1 << 20)) <= kSmemOptin;
 }
 static marie_status tall_cn(int64_t Nb, int M, int p, const cplx<float>* A, const cplx<float>* B, cplx<float>* H,
-                            cplx<float>* part, int* flag, cudaStream_t s) {
-  if (p <= 4) return tall_cn<4>(Nb, M, p, A, B, H, part, flag, s);
-  if (p <= 8) return tall_cn<8>(Nb, M, p, A, B, H, part, flag, s);
-  return tall_cn<16>(Nb, M, p, A, B, H, part, flag, s);
+                            cplx<float>* part, int64_t part_cap, int* flag, cudaStream_t s) {
+  if (p <= 4) return tall_cn<4>(Nb, M, p, A, B, H, part, part_cap, flag, s);
+  if (p <= 8) return tall_cn<8>(Nb, M, p, A, B, H, part, part_cap, flag, s);
+  return tall_cn<16>(Nb, M, p, A, B, H, part, part_cap, flag, s);
 }
 static marie_status tall_comb(int64_t Nb, int M, int p, float alpha, const cplx<float>* A, const cplx<float>* X,
                               float beta, cplx<float>* C, cudaStream_t s) {

@@ -728,7 +728,7 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
                                std::vector<RhsLog>& log, int* matvecs, cudaStream_t s, Scratch& sc) {
   const int64_t Nb = h->Nb;
   const int mp1 = m + 1;
-  const bool brief = short_vectors(Nb);
+  const bool brief = short_vectors(Nb) && h->mem_cap == 0;   // more partial sums
   const int per = brief ? kVTS : kCH;
   const int nch = (int)((Nb + per - 1) / per);
   const int nchd = brief ? (int)((Nb + kVTS * kDotVE - 1) / (kVTS * kDotVE)) : nch;   // of the projections
