@@ -228,7 +228,7 @@ marie_status marie_assemble_green(int32_t n1, int32_t n2, int32_t n3, double res
  * field inside a quasi-static dielectric sphere comes out ~3x too small. */
 #define MARIE_GREEN_SELF_POINT_TERM 1
 /* MARIE_GREEN_NEAR_EXACT replaces the near offsets {0,1}^3 (N or K) with an
- * accurate host cubature of the same integrals (relative coordinate
+ * accurate cubature of the same integrals (relative coordinate
  * u = r - r', the box split so that u = 0 is a corner of its pieces, Duffy
  * pyramids there, the static N singularity as a principal value over the
  * cube plus the point term above; converged to ~1e-14), instead of the
