@@ -1,4 +1,4 @@
-// Launch code of the four-step matvec passes (matvec4.cuh, kz4.cuh).
+// Launch code of the four-step matvec passes (xy4c, xy4f, matvec4, kz4p, kz4f, kz4).
 //
 // The per-pass launchers (switch over NB = n/16) are declared here and
 // defined in fastpath_impl.cuh, so that one precision's kernels can be spread

@@ -186,7 +186,7 @@ marie_status launch_fast_chunk(marie_vie* h, int op, MvArgs<T>& a, int nb, cudaS
 marie_status build_spectra(marie_vie* h, const marie_vie_desc* d);
 
 // Per-application Tucker expansion (tucker.cu): keep the N operator's
-// factors at create; rebuild the complex64 full spectrum on `s`.
+// factors at create; rebuild the complex64 octant columns on `s`.
 marie_status tucker_keep_c64(marie_vie* h, const marie_tucker_block* tk);
 marie_status tucker_expand_c64(marie_vie* h, cudaStream_t s);
 

@@ -1,8 +1,7 @@
 // Four-step z pass of the matvec (n3 = 16*NB): z-DFT, Green block multiply
 // and inverse z-DFT in shared memory, for W = TX*R contiguous elements of
 // every (component, z) row.  k4_z serves native complex128; complex64 and
-// float-float complex128 run the packed-pair kernels of kz4p.cuh and
-// kz4f.cuh, which keep this layout and work split.
+// float-float complex128 have kernels of their own (kz4p.cuh, kz4f.cuh).
 //
 // Shared-memory layout.  Half h (0: even frequencies, 1: odd) starts at
 // h*H; in it, sequence (c, e) starts at (c*W + e)*S.  Inside a sequence the
@@ -30,7 +29,7 @@ __device__ __forceinline__ cplx<double> shfl_xor_c(cplx<double> v, int m) {
 
 // One entry of the single-point Green multiply (entries sorted by block;
 // every index a compile-time constant).  gp points at the point's U block
-// values, contiguous in the full spectrum ([ky][kx][kz][blk], mirror signs
+// values, contiguous in the octant columns ([ky][kx][kz][blk], mirror signs
 // applied), so block blk sits at the constant offset blk.
 template <typename T, bool PWL, int OP, int K>
 struct ZPoint {

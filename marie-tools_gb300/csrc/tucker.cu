@@ -4,7 +4,7 @@
 //
 // With precisions bit 8 (MARIE_PREC_TUCKER_PER_APPLY) a handle built from
 // Tucker blocks keeps their factors on the device in FP32 and rebuilds the
-// complex64 full spectrum (the pair layout the four-step z pass reads) at the
+// complex64 octant columns (the pair layout the four-step z pass reads) at the
 // start of every complex64 application of N or N^H, once for all the chunks
 // of right-hand sides of that application:
 //   P1[a, b, kz] = sum_c G[a, b, c] U3[c, kz]             (r1 r2 x 2n3)
