@@ -206,13 +206,15 @@ def solve_alg_bytes(n, pwl, Nb, iters, n_c128, chunk, restart=50, block_steps=0,
 
 
 def roofline_z(op, wl, tiles, ms_z, peak, peak_kind, zfrac=1.0):
-    """Algorithmic bytes of one z-pass launch / its event-timed duration.
+    """Algorithmic bytes of the z pass of one chunk of right-hand sides / its
+    event-timed duration ms_z (over all its launches: an odd count goes as
+    powers of two on large grids).
     zfrac: fraction of z slices holding body voxels (the pass reads and
     writes those only)."""
     n, C = wl["n"], 12 if wl["pwl"] else 3
     U = 60 if wl["pwl"] else 6
     s = 8                                   # complex64
-    units = min(tiles["chunk"], wl["nrhs"])  # right-hand sides per launch
+    units = min(tiles["chunk"], wl["nrhs"])  # right-hand sides of ms_z
     per_rhs = 8 * n ** 3 * C * s * zfrac    # read + write 4 n^3 per component (live slices)
     green = U * (n + 1) ** 3 * s            # octant spectrum, read once per launch
     alg = units * per_rhs + green

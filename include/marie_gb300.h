@@ -348,7 +348,8 @@ marie_status marie_svie_pfft_destroy(marie_svie_pfft* h);
 /* Diagnostics. */
 /* Average device time [ms] of each matvec pass over `reps` repetitions of
  * one mvp_vie application of nrhs right-hand sides (x/y: device, precision
- * prec), timed with CUDA events on `stream`:
+ * prec), summed over the chunks the application runs in, timed with CUDA
+ * events on `stream`:
  * ms[0] x-forward, ms[1] y-forward, ms[2] z (FFT, Green multiply, iFFT),
  * ms[3] y-inverse, ms[4] x-inverse + epilogue.  ms[5] = whole application. */
 marie_status marie_vie_profile(marie_vie* h, int32_t prec, const void* x, void* y, int32_t nrhs, int32_t reps,

@@ -419,10 +419,29 @@ static marie_status alloc_workspace(marie_vie* h, PrecState<T>& ps) {
   return MARIE_OK;
 }
 
+// Events around the five passes, six per chunk of right-hand sides, kept from one
+// application to the next.
+struct PassEvents {
+  std::vector<cudaEvent_t> ev;
+  size_t used = 0;
+  cudaEvent_t* next() {
+    used += 6;
+    while (ev.size() < used) {
+      cudaEvent_t e = nullptr;
+      cudaEventCreate(&e);
+      ev.push_back(e);
+    }
+    return ev.data() + used - 6;
+  }
+  ~PassEvents() {
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  }
+};
+
 template <typename T>
 static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<typename IoOf<T>::type>* in,
                                      int64_t in_rs, cplx<typename IoOf<T>::type>* out, int64_t out_rs, int nrhs,
-                                     const unsigned char* active, cudaStream_t stream, cudaEvent_t* ev,
+                                     const unsigned char* active, cudaStream_t stream, PassEvents* prof,
                                      const cplx<typename IoOf<T>::type>* addend = nullptr);
 
 template <typename T, bool PWL, int OP>
@@ -464,11 +483,11 @@ marie_status launch_matvec(marie_vie* h, int mode, int op, const cplx<T>* in, in
   return launch_matvec_ev<T>(h, mode, op, in, in_rs, out, out_rs, nrhs, active, stream, nullptr);
 }
 
-// ev (optional): 6 events recorded around the 5 passes of the first chunk.
+// prof (optional): events recorded around the five passes of every chunk.
 template <typename T>
 static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<typename IoOf<T>::type>* in,
                                      int64_t in_rs, cplx<typename IoOf<T>::type>* out, int64_t out_rs, int nrhs,
-                                     const unsigned char* active, cudaStream_t stream, cudaEvent_t* ev,
+                                     const unsigned char* active, cudaStream_t stream, PassEvents* prof,
                                      const cplx<typename IoOf<T>::type>* addend) {
   PrecState<T>& ps = prec_state<T>(h);
   if (!ps.built) {
@@ -544,9 +563,10 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
     a.out = out + (int64_t)r0 * out_rs;
     a.active = active ? active + r0 : nullptr;
     a.addend = addend ? addend + (int64_t)r0 * out_rs : nullptr;
+    cudaEvent_t* ev = prof ? prof->next() : nullptr;
     if (fast) {
       a.G = isK ? ps.GKf : ps.GNf;
-      MARIE_TRY(launch_fast_chunk<T>(h, op, a, nb, stream, (ev && r0 == 0) ? ev : nullptr));
+      MARIE_TRY(launch_fast_chunk<T>(h, op, a, nb, stream, ev));
       continue;
     }
     if constexpr (std::is_same<T, ff>::value) {
@@ -560,23 +580,22 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
     dim3 gx((n2 + a.TY - 1) / a.TY, n3, nb * C);
     dim3 gy((2 * n1 + a.TXY - 1) / a.TXY, n3, nb * C);
     dim3 gz((2 * n1 + a.TX - 1) / a.TX, 2 * n2, nb);
-    const bool rec = ev && r0 == 0;
-    if (rec) cudaEventRecord(ev[0], stream);
+    if (ev) cudaEventRecord(ev[0], stream);
     k_fwd_x<T><<<gx, 256, smx, stream>>>(a);
     MARIE_LAUNCH_CHECK();
-    if (rec) cudaEventRecord(ev[1], stream);
+    if (ev) cudaEventRecord(ev[1], stream);
     k_fwd_y<T><<<gy, 256, smy, stream>>>(a);
     MARIE_LAUNCH_CHECK();
-    if (rec) cudaEventRecord(ev[2], stream);
+    if (ev) cudaEventRecord(ev[2], stream);
     dispatch_z<T>(h->pwl != 0, op, a, gz, smz, stream);
     MARIE_LAUNCH_CHECK();
-    if (rec) cudaEventRecord(ev[3], stream);
+    if (ev) cudaEventRecord(ev[3], stream);
     k_inv_y<T><<<gy, 256, smy, stream>>>(a);
     MARIE_LAUNCH_CHECK();
-    if (rec) cudaEventRecord(ev[4], stream);
+    if (ev) cudaEventRecord(ev[4], stream);
     k_inv_x<T><<<gx, 256, smx, stream>>>(a);
     MARIE_LAUNCH_CHECK();
-    if (rec) cudaEventRecord(ev[5], stream);
+    if (ev) cudaEventRecord(ev[5], stream);
     }
   }
   return MARIE_OK;
@@ -1073,36 +1092,38 @@ marie_status marie_vie_profile(marie_vie* h, int32_t prec, const void* x, void* 
   if (!h || !x || !y || !ms || nrhs < 1 || reps < 1) { set_error("marie_vie_profile: invalid argument"); return MARIE_ERR_BAD_ARG; }
   if (prec != MARIE_C128 && prec != MARIE_C64) { set_error("prec must be MARIE_C128 or MARIE_C64"); return MARIE_ERR_BAD_ARG; }
   cudaStream_t s = (cudaStream_t)stream;
-  cudaEvent_t ev[6], t0, t1;
-  for (int i = 0; i < 6; ++i) cudaEventCreate(&ev[i]);
+  PassEvents ev;
+  for (int i = 0; i < std::min(nrhs, 16); ++i) ev.next();   // not while the passes run
+  cudaEvent_t t0, t1;
   cudaEventCreate(&t0);
   cudaEventCreate(&t1);
   double acc[6] = {0, 0, 0, 0, 0, 0};
   marie_status st = MARIE_OK;
   for (int r = 0; r < reps && st == MARIE_OK; ++r) {
+    ev.used = 0;
     cudaEventRecord(t0, s);
     if (prec == MARIE_C128 && c128_is_ff(h))
       st = launch_matvec_ev<ff>(h, MV_VIE, OP_N, (const cplx<double>*)x, h->Nb, (cplx<double>*)y, h->Nb, nrhs,
-                                nullptr, s, ev);
+                                nullptr, s, &ev);
     else if (prec == MARIE_C128)
       st = launch_matvec_ev<double>(h, MV_VIE, OP_N, (const cplx<double>*)x, h->Nb, (cplx<double>*)y, h->Nb, nrhs,
-                                    nullptr, s, ev);
+                                    nullptr, s, &ev);
     else
       st = launch_matvec_ev<float>(h, MV_VIE, OP_N, (const cplx<float>*)x, h->Nb, (cplx<float>*)y, h->Nb, nrhs,
-                                   nullptr, s, ev);
+                                   nullptr, s, &ev);
     cudaEventRecord(t1, s);
     if (cudaEventSynchronize(t1) != cudaSuccess) { set_error("profile: device error"); st = MARIE_ERR_CUDA; break; }
-    for (int i = 0; i < 5; ++i) {
-      float v = 0;
-      cudaEventElapsedTime(&v, ev[i], ev[i + 1]);
-      acc[i] += v;
-    }
+    for (size_t c = 0; st == MARIE_OK && c < ev.used; c += 6)
+      for (int i = 0; i < 5; ++i) {
+        float v = 0;
+        cudaEventElapsedTime(&v, ev.ev[c + i], ev.ev[c + i + 1]);
+        acc[i] += v;
+      }
     float w = 0;
     cudaEventElapsedTime(&w, t0, t1);
     acc[5] += w;
   }
   for (int i = 0; i < 6; ++i) ms[i] = acc[i] / reps;
-  for (int i = 0; i < 6; ++i) cudaEventDestroy(ev[i]);
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
   return st;

@@ -176,7 +176,8 @@ class VieOperator:
 
     def profile(self, x, reps=5):
         """Per-pass device times [ms] of mvp_vie on x (CUDA events on the
-        current stream): x-fwd, y-fwd, z, y-inv, x-inv, whole application."""
+        current stream), each over all its launches: x-fwd, y-fwd, z, y-inv,
+        x-inv, whole application."""
         import torch
         prec = C128 if x.dtype == torch.complex128 else C64
         y = torch.empty_like(x)
