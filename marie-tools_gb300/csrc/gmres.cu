@@ -731,7 +731,7 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
   const bool brief = short_vectors(Nb) && h->mem_cap == 0;   // more partial sums
   const int per = brief ? kVTS : kCH;
   const int nch = (int)((Nb + per - 1) / per);
-  const int nchd = brief ? (int)((Nb + kVTS * kDotVE - 1) / (kVTS * kDotVE)) : nch;   // of the projections
+  const int nchd = brief ? (int)((Nb + kVTS * kDotVE - 1) / (kVTS * kDotVE)) : nch;   // of the projections: at most 512, 8 KB of sums per basis vector
   // CTAs per chunk in the projections of short vectors
   auto jsplit = [&](int k) {
     return (unsigned)(brief ? std::max(1, std::min(k + 1, (int)(2048 / std::max<int64_t>(1, (int64_t)nchd * nrhs)))) : 1);
@@ -751,7 +751,7 @@ static marie_status gmres_core(marie_vie* h, int nrhs, cplx<T>* V, int m, zd* x,
   MARIE_TRY(sc.get(&st.kr, nrhs));
   MARIE_TRY(sc.get(&st.hist, (size_t)nrhs * m));
   MARIE_TRY(sc.get(&st.incyc, nrhs));
-  MARIE_TRY(sc.get(&st.part, (size_t)nrhs * mp1 * nch));
+  MARIE_TRY(sc.get(&st.part, (size_t)nrhs * mp1 * nchd));
   MARIE_TRY(sc.get(&st.npart, (size_t)nrhs * nch));
   unsigned char* d_mask = nullptr;
   MARIE_TRY(sc.get(&d_mask, nrhs));
