@@ -16,6 +16,7 @@ namespace marie {
 
 typedef cplx<double> zd;
 
+// The kernels without their factor 1/(4 pi), which the callers' weights carry.
 // G_N.m entries [-Gyy-Gzz, Gxy, Gxz, -Gxx-Gzz, Gyz, -Gxx-Gyy]
 __device__ __forceinline__ void gn_kernel(double dx, double dy, double dz, double k0, zd* f) {
   const double R2 = dx * dx + dy * dy + dz * dz;
@@ -24,8 +25,7 @@ __device__ __forceinline__ void gn_kernel(double dx, double dy, double dz, doubl
   const double iR2 = iR * iR, iR3 = iR2 * iR, iR4 = iR2 * iR2, iR5 = iR4 * iR;
   double sn, cs;
   sin_cos(k0 * R, &sn, &cs);
-  const double q = 0.25 / 3.14159265358979323846;
-  const zd Ge = {cs * q, -sn * q};                 // exp(-i k0 R)/(4 pi)
+  const zd Ge = {cs, -sn};                         // exp(-i k0 R)
   const double k2 = k0 * k0;
   // diag: 3d^2/R^5 + 3i k0 d^2/R^4 - (1 + k0^2 d^2)/R^3 - i k0/R^2
   auto diag = [&](double d) -> zd {
@@ -43,14 +43,13 @@ __device__ __forceinline__ void gn_kernel(double dx, double dy, double dz, doubl
   f[5] = zd{-(xx.x + yy.x), -(xx.y + yy.y)};
 }
 
-// G_K.m entries [Gx, Gy, Gz] = exp(-ik0R)/(4pi) * (-d) * (1/R^3 + i k0/R^2)
+// G_K.m entries [Gx, Gy, Gz] = exp(-ik0R) * (-d) * (1/R^3 + i k0/R^2)
 __device__ __forceinline__ void gk_kernel(double dx, double dy, double dz, double k0, zd* f) {
   double R;
   const double iR = inv_sqrt(dx * dx + dy * dy + dz * dz, R);
   double sn, cs;
   sin_cos(k0 * R, &sn, &cs);
-  const double q = 0.25 / 3.14159265358979323846;
-  const zd Ge = {cs * q, -sn * q};
+  const zd Ge = {cs, -sn};
   const zd fac = Ge * zd{iR * iR * iR, k0 * iR * iR};
   f[0] = scale(fac, -dx);
   f[1] = scale(fac, -dy);
@@ -68,7 +67,12 @@ __device__ __forceinline__ void gk_kernel(double dx, double dy, double dz, doubl
 // kernel is evaluated at D^3 points instead of (n n')^3: 729 for 4096, 35937
 // for 262144.  The moments are then applied axis by axis: one thread per
 // (x, y) line sums its D kernel values over z with the three z weights, and
-// the CTA's outputs sum the lines with the x and y weights.
+// the CTA's outputs sum the lines with the x weights, row by row, and the rows with
+// the y weights.  Rows are summed in two parts and the sum over the rows carries
+// its rounding (two-sum), and the common factor is applied in two parts, so that
+// fewer points do not mean a larger error: 1.7e-16 and 1.9e-16 of a far offset's
+// values at 2 and 5 mm (3.8e-16 and 3.6e-16 with one running sum over the lines; the
+// sum over all point pairs 2.4e-16 and 2.2e-16).
 //
 // The sum is also symmetric under axis permutations (a permuted offset holds
 // the same values with components and moments permuted), so only offsets
@@ -76,7 +80,7 @@ __device__ __forceinline__ void gk_kernel(double dx, double dy, double dz, doubl
 //
 // Bound: FP64 arithmetic (two FMAs per clock and SM), almost all of it the
 // D^3 kernel values.  48^3 PWL, N, the whole call with its copy to the host:
-// 405 -> 9.9 ms (with k_near, which took 95 ms of it on the host).
+// 405 -> 9.8 ms (with k_near, which took 95 ms of it on the host).
 // ---------------------------------------------------------------------------
 struct AxisRule {
   const double* d;      // D differences X - X' on [-1, 1] nodes
@@ -84,7 +88,7 @@ struct AxisRule {
   int D;
 };
 constexpr int kVvThreads = 128;
-constexpr int kVvLines = 243;     // lines per pass: three offsets of the far rule (3 * 9^2), odd: conflict-free rows
+constexpr int kVvLines = 243;     // most lines per pass: three offsets of the far rule (3 * 9^2), odd: conflict-free rows
 
 enum WType { W_CC = 0, W_LC = 1, W_CL = 2, W_LL = 3 };
 // weight type of moment product j (VV_Nop.m:27-28) along axis d (0 x, 1 y, 2 z)
@@ -109,11 +113,12 @@ __host__ __device__ constexpr int perm_axis(int s, int d) {
 
 // offs: (a, b, c, rule | 8 * permute).  The first nspec blocks take one offset
 // each (medium rule and the near stand-in), the others three offsets of the
-// far rule.  out[(mx + n1(my + n2 mz)) + nD*(llp + pwx*comp)]
+// far rule.  J: (dx/2)^6 / (4 pi) in two parts (its rounding would be in every value).
+// out[(mx + n1(my + n2 mz)) + nD*(llp + pwx*comp)]
 template <int PWX, int NC, bool ISN>
 __global__ void __launch_bounds__(kVvThreads) k_vv(const int4* offs, int nspec, int noff, AxisRule r0, AxisRule r1,
-                                                   AxisRule r2, double dx, double k0, int n1, int n2, int n3,
-                                                   double* out) {
+                                                   AxisRule r2, double dx, double2 J, double k0, int n1, int n2,
+                                                   int n3, double* out) {
   extern __shared__ __align__(16) double vsm[];
   constexpr int NZ = PWX == 1 ? 1 : 3;          // z weight types in use: cc, cl, ll
   constexpr int NA = NZ * NC * 2;
@@ -132,12 +137,13 @@ __global__ void __launch_bounds__(kVvThreads) k_vv(const int4* offs, int nspec, 
   const double h = dx / 2;
   for (int i = threadIdx.x; i < 4 * D; i += kVvThreads) wt[i] = r.w[i];
   for (int i = threadIdx.x; i < D; i += kVvThreads) dd[i] = h * r.d[i];
-  double acc[PER];
+  double acc[PER], err[PER];
 #pragma unroll
-  for (int v = 0; v < PER; ++v) acc[v] = 0;
+  for (int v = 0; v < PER; ++v) acc[v] = err[v] = 0;
   const int total = cnt * D2;
-  for (int base = 0; base < total; base += kVvLines) {
-    const int nl = min(kVvLines, total - base);
+  const int pass = kVvLines / D * D;            // whole rows
+  for (int base = 0; base < total; base += pass) {
+    const int nl = min(pass, total - base);
     __syncthreads();
     for (int t = threadIdx.x; t < nl; t += kVvThreads) {
       const int o = (base + t) / D2, line = base + t - o * D2;
@@ -182,16 +188,23 @@ __global__ void __launch_bounds__(kVvThreads) k_vv(const int4* offs, int nspec, 
       const double* wy = wt + pair_type(j, 1) * D;
       const double* row = A + (((zt == W_CC ? 0 : (zt == W_CL ? 1 : 2)) * NC + c) * 2 + ri) * kVvLines;
       const int lo = max(o * D2 - base, 0), hi = min((o + 1) * D2 - base, nl);
-      double s = acc[v];
-      for (int t = lo; t < hi; ++t) {
-        const int line = base + t - o * D2;
-        const int iy = line / D, ix = line - iy * D;
-        s = fma(wx[ix] * wy[iy], row[t], s);
+      const int iy0 = (base + lo - o * D2) / D;
+      for (int t = lo, iy = iy0; t < hi; t += D, ++iy) {
+        double s0 = 0, s1 = 0;
+        int ix = 0;
+#pragma unroll 4
+        for (; ix + 1 < D; ix += 2) {
+          s0 = fma(wx[ix], row[t + ix], s0);
+          s1 = fma(wx[ix + 1], row[t + ix + 1], s1);
+        }
+        if (ix < D) s0 = fma(wx[ix], row[t + ix], s0);
+        const double r = s0 + s1, p = __dmul_rn(wy[iy], r);
+        const double sum = acc[v] + p, back = sum - acc[v];
+        err[v] += ((acc[v] - (sum - back)) + (p - back)) + fma(wy[iy], r, -p);
+        acc[v] = sum;
       }
-      acc[v] = s;
     }
   }
-  const double J = h * h * h * h * h * h;
   const int64_t nD = (int64_t)n1 * n2 * n3;
 #pragma unroll
   for (int v = 0; v < PER; ++v) {
@@ -215,7 +228,7 @@ __global__ void __launch_bounds__(kVvThreads) k_vv(const int4* offs, int nspec, 
       int cc;
       if (ISN) cc = comp_of(back(comp_p(c)), back(comp_q(c)));
       else cc = back(c);
-      out[2 * (mx + (int64_t)n1 * (my + (int64_t)n2 * mz) + nD * (jj + PWX * cc)) + ri] = acc[v] * J;
+      out[2 * (mx + (int64_t)n1 * (my + (int64_t)n2 * mz) + nD * (jj + PWX * cc)) + ri] = fma(acc[v], J.x, fma(acc[v], J.y, err[v] * J.x));
     }
   }
 }
@@ -263,12 +276,12 @@ __global__ void __launch_bounds__(kNearThreads) k_near(const double* gx, const d
   const double zero[3] = {0.0, 0.0, 0.0};
   double W0[PWX], W[PWX];
   weights(zero, W0);
-  const int f = (e + 1) % 3, g = (e + 2) % 3;
+  const int f = (e + 1) % 3;
   double acc = 0;
   const bool run = corner || e == 0;              // pieces away from 0 take one tensor rule
   for (int base = 0; run && base < kNearOrder * kNearOrder; base += kNearThreads) {
     const int j = (base + threadIdx.x) / kNearOrder, k = (base + threadIdx.x) - j * kNearOrder;
-    const double wq = gw[i] * gw[j] * gw[k] * vol;
+    const double wq = gw[i] * gw[j] * gw[k] * (vol * (0.25 / 3.14159265358979323846));
     zd Kf[NC], Ks[NC], Kt[NC];
     double u[3], ut[3];
     double c1 = wq, c2 = 0;
@@ -288,7 +301,6 @@ __global__ void __launch_bounds__(kNearThreads) k_near(const double* gx, const d
       c1 = wq * t * t;
       c2 = ISN ? wq / t : 0.0;
     }
-    (void)g;
     if (ISN) gn_kernel(u[0], u[1], u[2], k0, Kf);
     else gk_kernel(u[0], u[1], u[2], k0, Kf);
     if (ISN && corner) {
@@ -429,8 +441,10 @@ static cudaError_t run_vv(const int4* offs, int nspec, int noff, const DevRule* 
   }
   const int blocks = nspec + (noff - nspec + 2) / 3;
   if (blocks > 0) {
-    k_vv<PWX, NC, ISN><<<blocks, kVvThreads, smem>>>(offs, nspec, noff, rules[0].r, rules[1].r, rules[2].r, dx, k0, n1,
-                                                     n2, n3, out);
+    const long double h = 0.5L * dx, J = h * h * h * h * h * h / (4.0L * 3.141592653589793238462643383279502884L);
+    const double2 J2{(double)J, (double)(J - (double)J)};
+    k_vv<PWX, NC, ISN><<<blocks, kVvThreads, smem>>>(offs, nspec, noff, rules[0].r, rules[1].r, rules[2].r, dx,
+                                                     J2, k0, n1, n2, n3, out);
     g_launches++;
   }
   return cudaGetLastError();
