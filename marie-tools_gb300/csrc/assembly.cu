@@ -71,8 +71,8 @@ __device__ __forceinline__ void gk_kernel(double dx, double dy, double dz, doubl
 // the y weights.  Rows are summed in two parts and the sum over the rows carries
 // its rounding (two-sum), and the common factor is applied in two parts, so that
 // fewer points do not mean a larger error: 1.7e-16 and 1.9e-16 of a far offset's
-// values at 2 and 5 mm (3.8e-16 and 3.6e-16 with one running sum over the lines; the
-// sum over all point pairs 2.4e-16 and 2.2e-16).
+// values at 2 and 5 mm (with one running sum over the lines 3.8e-16 at 5 mm; the sum
+// over all point pairs 2.4e-16 and 2.2e-16).
 //
 // The sum is also symmetric under axis permutations (a permuted offset holds
 // the same values with components and moments permuted), so only offsets

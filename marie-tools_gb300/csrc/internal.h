@@ -184,6 +184,9 @@ template <typename T>
 marie_status launch_fast_chunk(marie_vie* h, int op, MvArgs<T>& a, int nb, cudaStream_t stream, cudaEvent_t* ev);
 
 marie_status build_spectra(marie_vie* h, const marie_vie_desc* d);
+// 1 / gain of the complex64 four-step transforms of an axis (0, 1, 2) at its octant
+// frequencies, which their spectrum carries (spectrum.cu).
+std::vector<double> four_step_inverse_gain(const marie_vie* h, int axis);
 
 // Per-application Tucker expansion (tucker.cu): keep the N operator's
 // factors at create; rebuild the complex64 octant columns on `s`.

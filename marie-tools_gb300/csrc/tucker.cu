@@ -111,6 +111,9 @@ marie_status tucker_keep_c64(marie_vie* h, const marie_tucker_block* tk) {
   const int nblk = h->nblkN;
   TuckerDev& t = h->tkf;
   t.blocks.assign(nblk, TuckerDev::Block{});
+  // the spectrum carries the inverse gain of the transforms (spectrum.cu)
+  const std::vector<double> gain[3] = {four_step_inverse_gain(h, 0), four_step_inverse_gain(h, 1),
+                                       four_step_inverse_gain(h, 2)};
   size_t mp1 = 1, mp2 = 1;
   const int m1 = 2 * h->n1, m2 = 2 * h->n2, m3 = 2 * h->n3;
   for (int id = 0; id < nblk; ++id) {
@@ -131,10 +134,15 @@ marie_status tucker_keep_c64(marie_vie* h, const marie_tucker_block* tk) {
     d.U3 = d.U2 + n2;
     std::vector<cplx<float>> host(ng + n1 + n2 + n3);
     const double* srcs[4] = {b.G, b.U1, b.U2, b.U3};
-    const size_t cnt[4] = {ng, n1, n2, n3};
+    const size_t cnt[4] = {ng, n1, n2, n3}, r[4] = {1, (size_t)b.r1, (size_t)b.r2, (size_t)b.r3};
+    const size_t n[4] = {1, (size_t)h->n1, (size_t)h->n2, (size_t)h->n3};
     size_t o = 0;
     for (int q = 0; q < 4; ++q)
-      for (size_t e = 0; e < cnt[q]; ++e, ++o) host[o] = cplx<float>{(float)srcs[q][2 * e], (float)srcs[q][2 * e + 1]};
+      for (size_t e = 0; e < cnt[q]; ++e, ++o) {
+        const size_t k = e / r[q];   // frequency of a factor's entry
+        const double g = q ? gain[q - 1][std::min(k, 2 * n[q] - k)] : 1.0;
+        host[o] = cplx<float>{(float)(srcs[q][2 * e] * g), (float)(srcs[q][2 * e + 1] * g)};
+      }
     MARIE_CUDA_TRY(cudaMemcpy(d.G, host.data(), host.size() * sizeof(cplx<float>), cudaMemcpyHostToDevice));
     mp1 = std::max(mp1, (size_t)b.r1 * b.r2 * m3);
     mp2 = std::max(mp2, (size_t)b.r1 * m2 * m3);
