@@ -383,7 +383,16 @@ static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, 
   }
   t.TX = std::max(1, std::min(2 * n1, Wz / t.R));
   // the complex64 PWL z pass shares each Green value among four elements
-  if (fast && sizeof(T) == 4 && h->pwl) t.TX = std::max(t.TX, 4 / t.R);
+  if (fast && sizeof(T) == 4) {
+    const int least = h->pwl ? std::max(4, t.R) : t.R;
+    t.TX = std::max(t.TX, least / t.R);
+    // narrower where all tiles still run at once: then a tile's latency counts (16^3 /
+    // 16 x 32 x 16 PWL, one right-hand side, z pass at W = 16 / 8 / 4: 16.0 / 13.0 /
+    // 11.9 and 22.2 / 16.1 / 17.4 us)
+    while (t.TX * t.R > least &&
+           kzp_tiles(n1, n2, t.TX * t.R / 2, t.R, (nr + t.R - 1) / t.R).total <= 2 * kSms)
+      t.TX /= 2;
+  }
   if (!fast) {   // generic passes: keep every tile within one CTA's shared memory
     const size_t sz = sizeof(cplx<T>);
     t.TY = std::min(t.TY, generic_tile_cap(h->n1, 1, t.R, sz));

@@ -6,6 +6,8 @@
 // kernels: x and y passes in two units, the z pass in one object per NB).
 #pragma once
 
+#include <algorithm>
+
 #include "internal.h"
 
 namespace marie {
@@ -50,7 +52,7 @@ __host__ __device__ constexpr int zp_freq(int NB, int p) { return zp_outer(NB) =
 // Tiles of the complex64 z pass (k4_zp): W = TX*R elements are, from the
 // lowest bit up, R right-hand sides, then the x mirror, then the y mirror,
 // then neighbouring columns, as far as W reaches; mirrors that do not fit
-// are tiles of their own.  At most two CTAs per SM, each walking the tiles.
+// are tiles of their own.  As many CTAs as run at once, each walking the tiles.
 struct ZpTiles {
   int lgW, lgR, cols;       // cols: octant columns kx per tile
   bool mx, my;              // mirrors inside the tile
@@ -73,10 +75,15 @@ __host__ __device__ inline ZpTiles kzp_tiles(int n1, int n2, int W, int R, int n
   return t;
 }
 constexpr int kSms = 152;
+// Threads of k4_zp: 512 an SM at 128 registers, in CTAs of 256; PWC of n3 = 16 has 48
+// tasks a tile and takes CTAs of 64 (16 x 32 x 16, sixteen right-hand sides: z pass
+// 36.2 -> 20.3 us).  Tiles that run at once.
+__host__ __device__ constexpr int zp_threads(int NB, bool pwl) { return NB == 1 && !pwl ? 64 : 256; }
+__host__ __device__ constexpr int zp_slots(int NB, bool pwl) { return kSms * (512 / zp_threads(NB, pwl)); }
 template <typename T>
 inline unsigned kzp_grid(const MvArgs<T>& a, int nb) {
   const int tiles = kzp_tiles(a.n1, a.n2, a.TX * a.R, a.R, nb).total;
-  return (unsigned)(tiles < 2 * kSms ? tiles : 2 * kSms);
+  return (unsigned)std::min(tiles, zp_slots(a.n3 / 16, a.C == 12));
 }
 
 template <typename T>

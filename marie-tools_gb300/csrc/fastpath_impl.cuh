@@ -76,7 +76,7 @@ static void launch_z4(const MvArgs<T>& a, dim3 g, size_t smem, cudaStream_t s) {
   static std::atomic<uint64_t> o{0};
   if constexpr (std::is_same<T, float>::value) {
     smem_opt_in(k4_zp<NB, PWL, OP>, o);
-    k4_zp<NB, PWL, OP><<<g, kZpThreads, smem, s>>>(a);
+    k4_zp<NB, PWL, OP><<<g, zp_threads(NB, PWL), smem, s>>>(a);
   } else if constexpr (std::is_same<T, ff>::value) {
     smem_opt_in(k4_zf<NB, PWL, OP>, o);
     k4_zf<NB, PWL, OP><<<g, kZfThreads, smem, s>>>(a);
