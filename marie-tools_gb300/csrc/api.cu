@@ -300,7 +300,7 @@ static marie_status choose_tiles(marie_vie* h, PrecState<T>& ps) {
 constexpr double kPadVolume = 3.0;    // see pad_c64
 
 struct CallTiles {
-  int R, TY, TXY, TX, TZY;
+  int R, TY, TXY, TX, WY;
 };
 
 // Bundle size R of nr right-hand sides: a power of two, <= the z tile width Wz.  The
@@ -361,25 +361,27 @@ static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, 
   const int wxy = (sizeof(T) == 4 ? 16 : 8) * (fast ? 2 : 1);   // row-tile width of the x/y passes
   t.TY = std::max(1, std::min(n2, wxy / t.R));
   t.TXY = std::max(1, std::min(2 * n1, wxy / t.R));
-  t.TZY = 1;
+  t.WY = 1;
   if (fast && sizeof(T) == 4) {
-    // slices of a column (xy4c.cuh): W = 32 elements per tile.  On short axes,
-    // where a tile's W*n/16 tasks leave most of 256 threads idle, more, while
-    // three tiles fit an SM and the CTAs make several waves (32 x 16 x 128 PWC,
-    // 22 right-hand sides: the four passes 253 -> 156 us; at 96^3 64 elements
-    // would slow the y pass 207 -> 243 us).  Fewer where 32 make less than a wave.
-    const int nb = (nr + t.R - 1) / t.R;
-    auto tile = [&](int n, int64_t lines) {
-      auto ctas = [&](int w) { return lines * nb * h->C * ((h->n3 * t.R + w - 1) / w); };
+    // W = 32 elements per tile (xy4c.cuh): slices of a row in the x passes, anything of
+    // a row in the y passes.  On short axes, where a tile's W*n/16 tasks leave most of
+    // 256 threads idle, more, while three tiles fit an SM and the CTAs make several
+    // waves (32 x 16 x 128 PWC, 22 right-hand sides: the four passes 253 -> 156 us; at
+    // 96^3 64 elements would slow the y pass 207 -> 243 us).  Fewer where 32 make less
+    // than a wave.
+    const int64_t nb = (nr + t.R - 1) / t.R;
+    auto tile = [&](int n, int64_t lines, int64_t line) {
+      auto ctas = [&](int w) { return lines * nb * h->C * ((line + w - 1) / w); };
       int w = std::max(wxy, t.R);
-      while (w * (n / 16) < 256 && (size_t)4 * w * (n + 1) * sizeof(cplx<T>) <= 72 * 1024 && w < 128 &&
-             w < h->n3 * t.R && ctas(2 * w) >= 4 * kSms)
+      while (w * (n / 16) < 256 && (size_t)4 * w * (n + 1) * sizeof(cplx<T>) <= 72 * 1024 && w < 128 && w < line &&
+             ctas(2 * w) >= 4 * kSms)
         w *= 2;
       while (w > std::max(8, t.R) && ctas(w) < kSms) w /= 2;
-      return w / t.R;
+      return w;
     };
-    t.TY = tile(n1, h->n2);
-    t.TZY = tile(n2, 2 * (int64_t)n1);
+    const int64_t col = (int64_t)h->n3 * t.R;
+    t.TY = tile(n1, h->n2, col) / t.R;
+    t.WY = tile(n2, 1, 2 * n1 * col);
   }
   t.TX = std::max(1, std::min(2 * n1, Wz / t.R));
   // the complex64 PWL z pass shares each Green value among four elements
@@ -566,7 +568,7 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
     a.TY = ct.TY;
     a.TXY = ct.TXY;
     a.TX = ct.TX;
-    a.TZY = ct.TZY;
+    a.WY = ct.WY;
     a.nrhs = nr;
     a.in = in + (int64_t)r0 * in_rs;
     a.out = out + (int64_t)r0 * out_rs;

@@ -123,11 +123,15 @@ marie_status launch_fast_chunk(marie_vie* h, int op, MvArgs<T>& a, int nb, cudaS
     return std::is_same<T, ff>::value ? xyf_smem(n, w) : (n + (size_t)2 * w * (n + 1)) * sz;
   };
   const size_t smx = smxy(n1, a.TY * a.R);
-  const size_t smy = smxy(n2, (c64 ? a.TZY : a.TXY) * a.R);
+  const size_t smy = smxy(n2, c64 ? a.WY : a.TXY * a.R);
   const size_t smz = kz4_smem<T>(n3, C, a.TX * a.R);
-  // x: TY rows (complex64: slices) per tile; y: TXY kx of a row (complex64: TZY slices)
+  // x: TY rows (complex64: slices) per tile; y: TXY kx of a row (complex64: WY elements)
   dim3 gx(c64 ? (a.g3 + a.TY - 1) / a.TY : (a.g2 + a.TY - 1) / a.TY, c64 ? a.g2 : a.g3, nb * C);
-  dim3 gy(c64 ? (a.g3 + a.TZY - 1) / a.TZY : (2 * n1 + a.TXY - 1) / a.TXY, c64 ? 2 * n1 : a.g3, nb * C);
+  dim3 gy((2 * n1 + a.TXY - 1) / a.TXY, a.g3, nb * C);
+  if constexpr (c64) {
+    const int col = a.g3 * a.R;
+    gy = col % a.WY == 0 ? dim3(col / a.WY, 2 * n1, nb * C) : dim3((2 * n1 * col + a.WY - 1) / a.WY, 1, nb * C);
+  }
   dim3 gz(nb, (2 * n1 + a.TX - 1) / a.TX, 2 * n2);
   if constexpr (c64) gz = dim3(kzp_grid(a, nb));
   if (ev) cudaEventRecord(ev[0], stream);

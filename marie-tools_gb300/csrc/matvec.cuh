@@ -97,7 +97,7 @@ struct MvArgs {
   const uint16_t* rowq;
   const uint16_t* zq;
   int TY, TXY, TX;            // tile sizes of the X, Y, Z passes
-  int TZY;                    // slices per tile of the complex64 four-step Y passes
+  int WY;                     // elements per tile of the complex64 four-step Y passes
 };
 
 template <typename T>

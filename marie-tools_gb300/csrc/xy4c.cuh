@@ -1,12 +1,13 @@
 // Four-step x and y passes of the complex64 operator (n = 16*NB): the split of
 // matvec4.cuh on work arrays whose slices z are contiguous,
 //   T1[bundle][c][y][2n1][z][R],  S[bundle][c][2n2][2n1][z][R],
-// over the caller's rows y < g2 and slices z < g3.  Every tile is W = TZ*R
-// neighbouring (slice, right-hand side) elements of one row or column, so all
-// three transforms read and write runs of W elements (256 bytes at W = 32), and
-// a z-pass column is one contiguous run.  (With rows of kx in T1 and columns of
-// z in S one of the two sides of the y passes had runs of 64 bytes: 128^3 PWL,
-// sixteen right-hand sides, 4.4 + 4.5 ms; now 3.5 + 4.1.)
+// over the caller's rows y < g2 and slices z < g3.  Every tile is W neighbouring
+// elements, (slice, right-hand side) of one row in the x passes, (kx, slice,
+// right-hand side) in the y passes, so all three transforms read and write runs of W
+// elements (256 bytes at W = 32), and a z-pass column is one contiguous run.  (With
+// rows of kx in T1 and columns of z in S one of the two sides of the y passes had runs
+// of 64 bytes: 128^3 PWL, every slice live, sixteen right-hand sides, 4.4 + 4.5 ms; now
+// 3.5 + 4.1.)
 //
 // Both halves of a zero-padded transform (even and odd frequencies) run in the
 // two lanes of packed FP32 pairs (pair.cuh), one instruction for both, and pass
@@ -272,13 +273,34 @@ __global__ void __launch_bounds__(256, 2) k4c_inv_x(MvArgs<float> a) {
 }
 
 // ---------------------------------------------------------------------------
-// Pass Y (forward).  grid (ceil(g3/TZ), 2n1, nbundle*C): the slices of a column
-// run back to back
+// Pass Y (forward).  The elements (kx, z, r) of a row lie back to back and a tile takes
+// WY of them: grid (g3*R / WY, 2n1, nbundle*C) where WY divides a column, else
+// (ceil(2n1*g3*R / WY), 1, nbundle*C), wherever columns begin, so that a short or ragged
+// z edge leaves no tile half empty (in tiles of one column's slices 64 x 16 x 16 PWL,
+// one right-hand side, Y 16.8, YI 18.4 us; now 12.4 and 12.4).  The first form saves the
+// division by g3 (96^3: 2% of the pass).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool y_tile_live(const MvArgs<float>& a, int z0, int tz) {
-  for (int i = 0; i < tz; ++i)
-    if (z_is_live(a, z0 + i)) return true;
-  return false;
+// The tile's first element of the row and whether any of its slices holds body voxels;
+// the thread's slice z (-1: none, or without body voxels).
+__device__ __forceinline__ bool y_tile(const MvArgs<float>& a, int& f0, int& z) {
+  const int q = blockIdx.x * a.WY, e = threadIdx.x & (a.WY - 1);   // WY divides the block size
+  int first = q >> a.lgR;
+  if (gridDim.y > 1) {     // whole tiles in a column, blockIdx.y: the column
+    f0 = blockIdx.y * a.g3 * a.R + q;
+    z = first + (e >> a.lgR);
+  } else {
+    f0 = q;
+    first %= a.g3;
+    z = (first + (e >> a.lgR)) % a.g3;
+    if (q + e >= 2 * a.n1 * a.g3 * a.R) z = -1;
+  }
+  bool any = false;
+  for (int i = 0, s = first; i < a.WY && !any; i += a.R) {
+    any = z_is_live(a, s);
+    if (++s == a.g3) s = 0;
+  }
+  if (z >= 0 && !z_is_live(a, z)) z = -1;
+  return any;
 }
 
 // One half at a time in scalar arithmetic at 80 registers: the pass waits for
@@ -289,26 +311,24 @@ __global__ void __launch_bounds__(256, 3) k4c_fwd_y(MvArgs<float> a) {
   constexpr int N = 16 * NB, S = N + 1;
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
   if (!bundle_active(a, bu)) return;
-  const int g2 = a.g2, g3 = a.g3, m1 = 2 * a.n1, R = a.R;
-  const int z0 = blockIdx.x * a.TZY, tz = min(a.TZY, g3 - z0);
-  if (!y_tile_live(a, z0, tz)) return;   // slices without body voxels: the z pass reads them as zero
-  const int W = a.TZY * R, lgW = 31 - __clz(W);
+  int f0, z;
+  if (!y_tile(a, f0, z)) return;   // slices without body voxels: the z pass reads them as zero
+  const int g2 = a.g2, W = a.WY, lgW = 31 - __clz(W);
   const XySmem sm = xy_smem(a.ay.tw, N);
   const cplx<float>* tw = sm.tw;
   cplx<float>* buf = reinterpret_cast<cplx<float>*>(sm.buf);   // half beta of sequence e at (beta*W + e)*S
-  const int e = threadIdx.x & (W - 1), z = z0 + (e >> a.lgR);   // W divides the block size
-  const bool ok = (e >> a.lgR) < tz && z_is_live(a, z);
+  const int e = threadIdx.x & (W - 1);
   __syncthreads();
-  const int64_t col = (int64_t)g3 * R, plane = m1 * col;
-  const cplx<float>* src = a.T1 + ((int64_t)bu * a.C + c) * g2 * plane + blockIdx.y * col + (int64_t)z0 * R + e;
+  const int64_t plane = (int64_t)2 * a.n1 * a.g3 * a.R;
   // step 1: task (b, e), e fastest
   for (int t = threadIdx.x; t < W * NB; t += blockDim.x) {
     const int b = t >> lgW;
-    const unsigned live = !ok ? 0u : (a.rowq ? a.rowq[z * 8 + b] : inside_bits(g2, NB, b));   // rows y = NB*q + b
+    const unsigned live = z < 0 ? 0u : (a.rowq ? a.rowq[z * 8 + b] : inside_bits(g2, NB, b));   // rows y = NB*q + b
+    const cplx<float>* src = a.T1 + ((int64_t)bc * g2 + b) * plane + f0 + e;
     cplx<float> v[16], u[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
-      const cplx<float> val = ((live >> q) & 1u) ? src[(NB * q + b) * plane] : cplx<float>{0, 0};
+      const cplx<float> val = ((live >> q) & 1u) ? src[NB * q * plane] : cplx<float>{0, 0};
       v[q] = val;
       u[q] = val;
     }
@@ -323,7 +343,7 @@ __global__ void __launch_bounds__(256, 3) k4c_fwd_y(MvArgs<float> a) {
   }
   __syncthreads();
   // step 2: task (beta, k1, e), e fastest; ky' = beta*N + k
-  cplx<float>* dst = a.S + ((int64_t)bu * a.C + c) * 2 * N * plane + blockIdx.y * col + (int64_t)z0 * R + e;
+  cplx<float>* dst = a.S + (int64_t)bc * 2 * N * plane + f0 + e;
   for (int t = threadIdx.x; t < 2 * 16 * W; t += blockDim.x) {
     const int q = t >> lgW;
     const int k1 = q & 15, beta = q >> 4;
@@ -331,7 +351,7 @@ __global__ void __launch_bounds__(256, 3) k4c_fwd_y(MvArgs<float> a) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) w[b] = buf[(beta * W + e) * S + k1 * NB + b];
     dftn<float, false, NB>(w);
-    if (ok) {
+    if (z >= 0) {
       cplx<float>* o = dst + (beta * N + k1) * plane;
 #pragma unroll
       for (int k2 = 0; k2 < NB; ++k2) o[16 * k2 * plane] = w[k2];
@@ -347,28 +367,26 @@ __global__ void __launch_bounds__(256, 2) k4c_inv_y(MvArgs<float> a) {
   constexpr int N = 16 * NB, S = N + 1;
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
   if (!bundle_active(a, bu)) return;
-  const int g2 = a.g2, g3 = a.g3, m1 = 2 * a.n1, R = a.R;
-  const int z0 = blockIdx.x * a.TZY, tz = min(a.TZY, g3 - z0);
-  if (!y_tile_live(a, z0, tz)) return;   // no body voxel in these slices: no output
-  const int W = a.TZY * R, lgW = 31 - __clz(W);
+  int f0, z;
+  if (!y_tile(a, f0, z)) return;   // no body voxel in these slices: no output
+  const int g2 = a.g2, W = a.WY, lgW = 31 - __clz(W);
   const XySmem sm = xy_smem(a.ay.tw, N);
-  const int e = threadIdx.x & (W - 1), z = z0 + (e >> a.lgR);
-  const bool ok = (e >> a.lgR) < tz && z_is_live(a, z);
+  const int e = threadIdx.x & (W - 1);
   __syncthreads();
-  const int64_t col = (int64_t)g3 * R, plane = m1 * col;
-  const cplx<float>* src = a.S + ((int64_t)bu * a.C + c) * 2 * N * plane + blockIdx.y * col + (int64_t)z0 * R + e;
+  const int64_t plane = (int64_t)2 * a.n1 * a.g3 * a.R;
+  const cplx<float>* src = a.S + ((int64_t)bu * a.C + c) * 2 * N * plane + f0 + e;
   // step A: task (k1, e): inverse NB-point DFT over k2, twiddle
-  for (int t = threadIdx.x; t < 16 * W && ok; t += blockDim.x) {
+  for (int t = threadIdx.x; t < 16 * W && z >= 0; t += blockDim.x) {
     const int k1 = t >> lgW;
     const cplx<float>* in = src + k1 * plane;
     pair_invn<NB>(sm.buf + e * S + k1 * NB, in, in + N * plane, 16 * plane, k1, sm.tw);
   }
   __syncthreads();
   // step B: task (b, e): inverse 16-point DFTs of both halves, combine, store
-  cplx<float>* dst = a.T1 + ((int64_t)bu * a.C + c) * g2 * plane + blockIdx.y * col + (int64_t)z0 * R + e;
+  cplx<float>* dst = a.T1 + ((int64_t)bu * a.C + c) * g2 * plane + f0 + e;
   for (int t = threadIdx.x; t < W * NB; t += blockDim.x) {
     const int b = t >> lgW;
-    const unsigned live = !ok ? 0u : (a.rowq ? a.rowq[z * 8 + b] : inside_bits(g2, NB, b));   // rows y = NB*q + b
+    const unsigned live = z < 0 ? 0u : (a.rowq ? a.rowq[z * 8 + b] : inside_bits(g2, NB, b));   // rows y = NB*q + b
     if (!live) continue;
     cplx<float> v[16];
     pair_inv16<NB>(v, sm.buf + e * S + b, b, a.ay.tw2);
