@@ -305,20 +305,26 @@ struct CallTiles {
 
 // Bundle size R of nr right-hand sides: a power of two, <= the z tile width Wz.  The
 // last bundle computes its empty places too, so few of them come first; a wide
-// bundle shares each Green value and twiddle, worth a quarter of a product between
-// one and many in complex64, a sixteenth in the arithmetic-bound precisions (per
-// right-hand side at R = 1 / 2 / 4: 96^3 PWL complex64 880 / 818 / 796 us, 112^3 PWC
-// 303 / 274 / 253, 48^3 PWL 150 / 137 / 116, float-float 557 / 552 / 540).  Against
-// the largest R <= nr: 96^3 PWL five 6.37 -> 4.41 ms, three 3.27 -> 2.68; complex128
-// 33 x 30 x 28 PWL three 3.38 -> 2.68; seven stay at R = 4 in complex64 (112^3 PWC
-// 2.03 ms, 2.10 at R = 1).
+// bundle shares each Green value and twiddle: a bundle costs R + share places.
+// share (bundle_share): a sixteenth in the arithmetic-bound precisions, a quarter in
+// complex64 (per right-hand side at R = 1 / 2 / 4: 96^3 PWL complex64 880 / 818 / 796
+// us, 112^3 PWC 303 / 274 / 253, float-float 557 / 552 / 540).  A z edge of 16 or less
+// leaves the complex64 four-step x tiles (runs of slices and right-hand sides) half
+// empty: three quarters, and a bundle may be wider than nr (64 x 64 x 16 PWL, three in
+// one bundle of four 276 us, singly 304; five by two 451, singly 489, in one of eight
+// 501; at 90 x 90 x 18 three singly 768, in one of four 906).  Against the largest R <=
+// nr: 96^3 PWL five 6.37 -> 4.41 ms, three 3.27 -> 2.68; complex128 33 x 30 x 28 PWL
+// three 3.38 -> 2.68.
 template <typename T>
-static int bundle_size(int nr, int Wz, double* least = nullptr) {
-  const double share = sizeof(T) == 4 ? 0.25 : 0.0625;
+static double bundle_share(const marie_vie* h, bool fast) {
+  if (sizeof(T) != 4) return 0.0625;
+  return fast && h->n3 <= 16 ? 0.75 : 0.25;
+}
+static int bundle_size(int nr, int Wz, double share, bool wider, double* least = nullptr) {
   int best = 1;
   double lc = 0;
-  for (int R = 1; R <= Wz && R <= std::max(1, nr); R *= 2) {
-    const double cost = (double)((nr + R - 1) / R * R) * (1 + share / R);
+  for (int R = 1; R <= Wz && (wider ? R / 2 : R - 1) < std::max(1, nr); R *= 2) {
+    const double cost = (double)((nr + R - 1) / R) * (R + share);
     if (R == 1 || cost <= lc) {
       best = R;
       lc = cost;
@@ -335,16 +341,16 @@ static int bundle_size(int nr, int Wz, double* least = nullptr) {
 // 4.40, seven 5.80 / 6.42; 112^3 PWC seven 1.96 / 2.02; 60 x 77 x 90 PWL three 1.53 /
 // 1.55; but 64^3 PWL (3.1 million values) three 0.85 / 0.83, 48^3 PWL seven 0.96 / 0.93.
 constexpr int64_t kSplitElements = 1 << 22;
-static double split_cost(int nr, int Wz, int* first) {
+static double split_cost(int nr, int Wz, double share, int* first) {
   double whole;
-  bundle_size<float>(nr, Wz, &whole);
+  bundle_size(nr, Wz, share, false, &whole);
   *first = nr;
   int q = 1, rest;
   while (q * 2 <= nr) q *= 2;
   if (q == nr || q > Wz) return whole;
   double head;
-  bundle_size<float>(q, Wz, &head);
-  const double parts = head + split_cost(nr - q, Wz, &rest);
+  bundle_size(q, Wz, share, false, &head);
+  const double parts = head + split_cost(nr - q, Wz, share, &rest);
   if (parts > 0.95 * whole) return whole;
   *first = q;
   return parts;
@@ -356,7 +362,7 @@ template <typename T>
 static CallTiles call_tiles(const marie_vie* h, const PrecState<T>& ps, int nr, bool fast) {
   CallTiles t;
   const int Wz = ps.TX;
-  t.R = bundle_size<T>(nr, Wz);
+  t.R = bundle_size(nr, Wz, bundle_share<T>(h, fast), fast && sizeof(T) == 4);
   const int n1 = ps.m1, n2 = ps.m2;
   const int wxy = (sizeof(T) == 4 ? 16 : 8) * (fast ? 2 : 1);   // row-tile width of the x/y passes
   t.TY = std::max(1, std::min(n2, wxy / t.R));
@@ -559,7 +565,7 @@ static marie_status launch_matvec_ev(marie_vie* h, int mode, int op, const cplx<
   const bool fast = four_step_op(h, ps, op) && (ps.padded || !env_int("MARIE_GENERIC_FFT", 0));
   for (int r0 = 0, nr; r0 < nrhs; r0 += nr) {
     nr = std::min(ps.ws_rhs, nrhs - r0);
-    if (fast && sizeof(T) == 4 && (int64_t)C * n1 * n2 * n3 >= kSplitElements) split_cost(nr, ps.TX, &nr);
+    if (fast && sizeof(T) == 4 && (int64_t)C * n1 * n2 * n3 >= kSplitElements) split_cost(nr, ps.TX, bundle_share<T>(h, fast), &nr);
     const CallTiles ct = call_tiles(h, ps, nr, fast);
     const int nb = (nr + ct.R - 1) / ct.R;
     a.R = ct.R;
