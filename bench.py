@@ -232,8 +232,8 @@ def roofline_z(op, wl, tiles, ms_z, peak, peak_kind, zfrac=1.0):
         model = units * per_rhs + columns
         model96 = 4 * 8 * 96 ** 3 * 12 * 8 * Z96_LIVE + 60 * 97 ** 2 * 192 * 8
         traffic = int(model * (Z96_DRAM_BYTES / model96))
-    four_step = n % 16 == 0 and 16 <= n <= 128
-    name = (f"k4_zp<{n // 16},{'PWL' if wl['pwl'] else 'PWC'}>" if four_step else "k_z<float>")
+    four_step = n % 16 == 0 and 16 <= n <= 128 or tiles["padded"]
+    name = (f"k4_zp<{(n + 15) // 16},{'PWL' if wl['pwl'] else 'PWC'}>" if four_step else "k_z<float>")
     # FP32 work of the same launch: per right-hand side and (kx, ky) column,
     # C forward + C inverse zero-padded transforms (two n-point halves each,
     # 5 m log2 m flops per m-point transform, plus 6 flops per point for the

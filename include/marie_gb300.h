@@ -370,7 +370,10 @@ marie_status marie_vie_autotune(marie_vie* h, int32_t prec, const void* x, void*
                                 int32_t* widths, double* ms, int32_t cap, int32_t* count, void* stream);
 /* Workspace right-hand sides per matvec chunk and the z-pass tile width:
  * out[0] = chunk, out[1] = tile width (pencils x interleaved right-hand
- * sides), out[2..3] reserved (0). */
+ * sides), out[2] = 1 if prec runs in float-float arithmetic, out[3] = 1 if the
+ * complex64 transforms run padded to multiples of 16 (grids whose edges are
+ * not, where that is faster; MARIE_GENERIC_FFT=1 at create keeps them on the
+ * grid's own lengths, later it has no effect on such a handle). */
 marie_status marie_vie_tiles(marie_vie* h, int32_t prec, int32_t* out);
 const char* marie_last_error(void);
 const char* marie_version(void);

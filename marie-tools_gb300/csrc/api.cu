@@ -297,8 +297,6 @@ static marie_status choose_tiles(marie_vie* h, PrecState<T>& ps) {
   return MARIE_OK;
 }
 
-constexpr double kPadVolume = 3.0;    // see pad_c64
-
 struct CallTiles {
   int R, TY, TXY, TX, WY;
 };
@@ -730,34 +728,16 @@ static marie_status validate_desc(const marie_vie_desc* d, std::vector<int64_t>&
   return MARIE_OK;
 }
 
-// complex64 on a grid that is not 16*NB: run the four-step passes on the next
-// multiples of 16 (the operator is a convolution, so any circulant of size 2m >=
-// 2n - 1 with zeros at the offsets n..m-1 gives the same on the grid, embed.h;
-// rows, slices and columns beyond the grid are never stored or read).  The
-// generic passes take four to five times as long per grid point (60 x 77 x 90
-// PWL, three right-hand sides: 6.5 ms against 1.5; 24^3 PWL one: 91 against 81
-// us at 2.4 times the volume; 17 x 40 x 40 PWL four: 491 against 339 at 2.7), so
-// padding pays up to about three times the volume.  Not under a memory cap, nor
-// where the larger work arrays and spectra would not fit easily: the generic
-// passes need less.  MARIE_GENERIC_FFT=1 at create keeps the generic passes.
-static marie_status pad_c64(marie_vie* h, const std::vector<int64_t>& idxS) {
+// Four-step passes of the complex64 state on lengths rounded up to multiples of 16
+// where they pay (embed::pad_dims: a rule of the grid and the basis alone).  Not under
+// a memory cap (the generic passes need less) nor with MARIE_GENERIC_FFT=1 at create.
+static bool pad_wanted(const marie_vie_desc* d, int m[3]) {
+  const int n[3] = {d->n1, d->n2, d->n3};
+  return (d->precisions & 2) && d->mem_cap_bytes <= 0 && !env_int("MARIE_GENERIC_FFT", 0) &&
+         embed::pad_dims(n, d->basis == MARIE_PWL ? 12 : 3, m);
+}
+static marie_status pad_c64(marie_vie* h, const int m[3], const std::vector<int64_t>& idxS) {
   PrecState<float>& ps = h->p32;
-  if (four_step_grid(h) || h->mem_cap > 0 || env_int("MARIE_GENERIC_FFT", 0)) return MARIE_OK;
-  const int n[3] = {h->n1, h->n2, h->n3};
-  int m[3];
-  double vol = 1;
-  for (int d = 0; d < 3; ++d) {
-    if (n[d] > 128) return MARIE_OK;
-    m[d] = (n[d] + 15) / 16 * 16;
-    vol *= (double)m[d] / n[d];
-  }
-  if (vol > kPadVolume) return MARIE_OK;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); return MARIE_OK; }
-  const double rhs = std::max(1, std::min(h->max_rhs, env_int("MARIE_WS_RHS", 16))) + 16.0;
-  const double need = 8.0 * ((h->nblkN + (h->has_K ? h->nblkK : 0)) * (m[0] + 1.0) * (m[1] + 1.0) * 2.0 * m[2] +
-                             rhs * h->C * n[2] * (2.0 * m[0]) * (n[1] + 2.0 * m[1]));
-  if (need > 0.25 * (double)free_b) return MARIE_OK;
   ps.m1 = m[0];
   ps.m2 = m[1];
   ps.m3 = m[2];
@@ -774,8 +754,9 @@ static marie_status pad_c64(marie_vie* h, const std::vector<int64_t>& idxS) {
 }
 
 // Handle for a grid the FFT passes take as given (marie_vie_create decides
-// whether the caller's grid is first embedded in a larger one, embed.h).
-static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
+// whether the caller's grid is first embedded in a larger one, embed.h); pad: the
+// transform lengths of a padded complex64 state, or null.
+static marie_status create_lengths(marie_vie** out, const marie_vie_desc* d, const int* pad) {
   if (!out) { set_error("output handle pointer is NULL"); return MARIE_ERR_BAD_ARG; }
   *out = nullptr;
   std::vector<int64_t> idxS;
@@ -878,9 +859,7 @@ static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
   own_dims(h->p64);
   own_dims(h->pff);
   own_dims(h->p32);
-  if (d->precisions & 2) {
-    if ((st = pad_c64(h, idxS)) != MARIE_OK) return fail(st);
-  }
+  if (pad && (st = pad_c64(h, pad, idxS)) != MARIE_OK) return fail(st);
   for (int pr = 0; pr < 3; ++pr) {
     if (!(d->precisions & (1 << pr))) continue;
     if (pr == 2) {
@@ -933,6 +912,17 @@ static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
   }
   *out = h;
   return MARIE_OK;
+}
+
+// The padded state's arrays are up to twice the others': where the device has no room
+// for them, the same handle on the generic passes.
+static marie_status create_grid(marie_vie** out, const marie_vie_desc* d) {
+  int m[3];
+  if (d && pad_wanted(d, m)) {
+    const marie_status st = create_lengths(out, d, m);
+    if (st != MARIE_ERR_OOM) return st;
+  }
+  return create_lengths(out, d, nullptr);
 }
 
 // Autotuner of the z-pass tile width: time `reps` applications of mvp_vie
@@ -1167,7 +1157,7 @@ marie_status marie_vie_tiles(marie_vie* h, int32_t prec, int32_t* out) {
   if (!h || !out) { set_error("marie_vie_tiles: invalid argument"); return MARIE_ERR_BAD_ARG; }
   if (prec == MARIE_C128 && c128_is_ff(h)) { out[0] = h->pff.ws_rhs; out[1] = h->pff.TX; out[2] = 1; out[3] = 0; }
   else if (prec == MARIE_C128) { out[0] = h->p64.ws_rhs; out[1] = h->p64.TX; out[2] = 0; out[3] = 0; }
-  else { out[0] = h->p32.ws_rhs; out[1] = h->p32.TX; out[2] = 0; out[3] = 0; }
+  else { out[0] = h->p32.ws_rhs; out[1] = h->p32.TX; out[2] = 0; out[3] = h->p32.padded; }
   return MARIE_OK;
 }
 

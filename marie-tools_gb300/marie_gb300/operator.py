@@ -205,7 +205,7 @@ class VieOperator:
     def tiles(self, prec=C64):
         out = np.zeros(4, np.int32)
         check(self._lib.marie_vie_tiles(self._h, prec, out.ctypes.data_as(_lib.c_int32_p)))
-        return dict(chunk=int(out[0]), width=int(out[1]), float_float=bool(out[2]))
+        return dict(chunk=int(out[0]), width=int(out[1]), float_float=bool(out[2]), padded=bool(out[3]))
 
     # -- field post-processing -------------------------------------------------
     def fields(self, J, Ue=None, Ub=None, *, e=True, h=True):
