@@ -51,15 +51,15 @@ inline bool smooth31(int n) {
 // gives the same on the grid; rows, slices and columns beyond it are never stored or
 // read.  C = 3 (PWC) or 12 (PWL) components.
 //
-// x pass, y pass and z pass grow by a, a*b and a*b*c for edges padded by factors a, b, c,
-// and take some 15, 25 and 60 hundredths of a product.  110 random and 55 chosen grids
-// with volumes a*b*c of 1.1 to 3, both bases, 1, 2, 3, 5, 8 and 16 right-hand sides:
-// with that cost up to 2.45 padding is faster by 3.4x at most (96 x 96 x 6 PWC 2.5x, 24^3
-// PWL 1.2x, 24 x 24 x 20 PWC 1.07x on the average) and slower by 7% at most, on
-// products of 40 us; at x edges below 9 (8 x 64 x 64 PWC 0.87x) and below 24000 grid
-// values (16 x 8 x 16 PWC 0.87x) it is the launches and the short rows that count.  An
-// edge with a prime factor above 7 runs a general butterfly in the mixed-radix passes,
-// of more than twice the time: padded up to three times the volume (34^3 PWL 3.1x).
+// 110 random and 55 chosen grids, both bases, 1, 2, 3, 5, 8 and 16 right-hand sides:
+// where this says yes, padding is faster by 6% or more (up to 3.4x) on the average of a
+// grid's counts, and at single counts slower by 13% at most, on products of 40 us
+// (24 x 24 x 20 PWC one 0.93x, PWL 1.14x on the average; 34^3 PWL 3.1x).  Where the other
+// passes stay: three times the volume and more (20^3 PWL 0.98x, 20 x 20 x 36 PWL 0.88x
+// at three); x edges below 9, whose rows are short in all passes (6 x 64 x 64 PWC 0.98x,
+// 0.82x at three); below 18000 grid values, where the launches count (16 x 8 x 16 PWC
+// 0.97x), unless little is added.  An edge with a prime factor above 7 runs a general
+// butterfly in the mixed-radix passes, of more than twice the time.
 inline bool pad_dims(const int n[3], int C, int m[3]) {
   bool same = true, prime = false;
   for (int d = 0; d < 3; ++d) {
@@ -72,9 +72,9 @@ inline bool pad_dims(const int n[3], int C, int m[3]) {
     prime = prime || v > 1;
   }
   if (same) return false;
-  const double a = (double)m[0] / n[0], ab = a * m[1] / n[1], vol = ab * m[2] / n[2];
-  if (vol > 3.0) return false;
-  return prime || (n[0] >= 9 && (double)C * n[0] * n[1] * n[2] >= 24000 && 0.15 * a + 0.25 * ab + 0.6 * vol <= 2.45);
+  const double values = (double)C * n[0] * n[1] * n[2];
+  const double vol = (double)m[0] * m[1] * m[2] / ((double)n[0] * n[1] * n[2]);
+  return vol <= 3.0 && (prime || (n[0] >= 9 && (values >= 18000 || vol <= 1.5)));
 }
 
 // Grid the caller's n is embedded in; false when it runs as given.

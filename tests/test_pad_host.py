@@ -29,10 +29,11 @@ def pad(tmp_path_factory):
 
 PADDED = [((60, 77, 90), False), ((60, 77, 90), True), ((100, 100, 100), True), ((24, 24, 24), True), ((24, 24, 20), True),
           ((20, 40, 40), False), ((96, 96, 6), False), ((64, 64, 8), True), ((34, 34, 34), False), ((11, 30, 30), False),
-          ((22, 22, 30), False), ((127, 128, 128), True), ((13, 30, 45), False)]
+          ((22, 22, 30), False), ((127, 128, 128), True), ((13, 30, 45), False), ((20, 24, 24), True),
+          ((18, 20, 32), False), ((16, 16, 12), False), ((32, 32, 6), False)]
 OWN = [((64, 64, 64), True), ((16, 32, 128), False), ((8, 64, 64), False), ((8, 64, 64), True), ((6, 96, 96), True),
-       ((16, 8, 16), False), ((16, 16, 12), False), ((17, 17, 17), True), ((18, 18, 18), False), ((20, 20, 20), True),
-       ((129, 64, 64), False), ((144, 150, 150), True), ((10, 10, 10), False), ((20, 24, 24), True)]
+       ((16, 8, 16), False), ((16, 16, 8), False), ((17, 17, 17), True), ((18, 18, 18), False), ((20, 20, 20), True),
+       ((129, 64, 64), False), ((144, 150, 150), True), ((10, 10, 10), False), ((16, 16, 5), True)]
 
 
 @pytest.mark.parametrize("n,pwl", PADDED, ids=str)
