@@ -169,12 +169,15 @@ static std::vector<double> inverse_gain(int n, int live, bool zpass) {
   std::vector<double> w(2 * n);     // of w_2n^k
   for (int k = 0; k < 2 * n; ++k) w[k] = sq(pi * k / n);
   // factors of the small DFTs (dft16, and dft_small / dft6 of NB points): frequency k, input j
-  auto small16 = [&](int k, int j) { const int m = (k & 3) * (j & 3); return m & 3 ? sq(2 * pi * m / 16) : 1.0; };
-  auto prime = [&](int k, int j, int R) { const int m = j * k % R; return m ? sq(2 * pi * m / R) : 1.0; };
+  const int R = NB == 6 ? 3 : NB;
+  double m16[10], mr[8], m8 = sq(pi / 4), m6 = sq(pi / 3);
+  for (int m = 0; m < 10; ++m) m16[m] = m & 3 ? sq(2 * pi * m / 16) : 1.0;
+  for (int m = 0; m < 8; ++m) mr[m] = m % R ? sq(2 * pi * m / R) : 1.0;
+  auto small16 = [&](int k, int j) { return m16[(k & 3) * (j & 3)]; };
   auto smalln = [&](int k, int j) {
-    if (NB == 8) return (j & k & 1) ? sq(pi / 4) : 1.0;
-    if (NB == 6) return ((k & 1) && j % 3 ? sq(2 * pi / 6) : 1.0) * prime(k >> 1, j % 3, 3);
-    return NB == 3 || NB == 5 || NB == 7 ? prime(k, j, NB) : 1.0;
+    if (NB == 8) return (j & k & 1) ? m8 : 1.0;
+    if (NB == 6) return ((k & 1) && j % 3 ? m6 : 1.0) * mr[(k >> 1) * (j % 3) % 3];
+    return NB == 3 || NB == 5 || NB == 7 ? mr[j * k % NB] : 1.0;
   };
   const bool split_nb = zpass && zp_outer(NB) == NB;   // k4_zp: NB points first, 16 after the twiddles
   std::vector<double> g(2 * n, 0.0);
