@@ -1,5 +1,7 @@
-// Host-side additions to the Green's-tensor assembly (no CUDA): compiled
-// into the library by assembly.cu and, for CPU tests, by a g++ shim.
+// Host parts of the Green's-tensor assembly (no CUDA).  The library (assembly.cu) uses
+// the self point term, the rule on [0, 1] and the moment overlaps; the near zone as a
+// whole (kernel_at, moment_weights, near_zone_offset, near_zone_exact) is the host form
+// of k_near's cubature, compiled by the CPU tests, which pin the formulas without a GPU.
 #pragma once
 
 #include <algorithm>

@@ -96,7 +96,7 @@ __device__ __forceinline__ void dftn(cplx<T>* v) {
 // buf: sequence s = (yy*R + r)*2 + alpha, stride S = 16*NB + 1, [k1][b]
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_x(MvArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) k4_fwd_x(MvArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int N = 16 * NB, S = N + 1;
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_x(MvArgs<T
 // Pass XI (inverse x + crop + epilogue), n1 = 16*NB.
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) k4_inv_x(MvArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int N = 16 * NB, S = N + 1;
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_x(MvArgs<T
 // buf: sequence s = beta*W + e, stride S, [k1][b]
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_y(MvArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) k4_fwd_y(MvArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int N = 16 * NB, S = N + 1;
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_fwd_y(MvArgs<T
 // Pass YI (inverse y + crop), n2 = 16*NB.
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k4_inv_y(MvArgs<T> a) {
+__global__ void __launch_bounds__(256, 2) k4_inv_y(MvArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int N = 16 * NB, S = N + 1;
   const int bc = blockIdx.z, bu = bc / a.C, c = bc - bu * a.C;
