@@ -8,7 +8,7 @@
 // a GEMM's 128-wide tiles of a p-wide result are far from: 48^3 PWL, eight
 // right-hand sides, the emulated GEMMs took 0.8 ms for a step's projection and
 // update and 1.3 ms for its block QR, two and a half times the operator's 0.95
-// ms (the whole solve 947 -> 463 ms).  At 240 vectors of 396960 the two take 219 and
+// ms (the whole solve 947 -> 463 ms, on the operator of that time).  At 240 vectors of 396960 the two take 219 and
 // 228 us (HBM alone 116, the FP32 work alone 82): many loads in flight beside the
 // arithmetic are what counts, so few registers a thread, and sums over a warp that
 // exchange each value once (k_tall_cn with four columns a pass and a butterfly per

@@ -22,8 +22,9 @@
 // inputs enter and the outputs leave.
 //
 // Measured against the kernel before it (full spectrum, one tile per CTA, rows
-// of kx in S): 96^3 PWL one right-hand side 0.814 -> 0.532 ms, 128^3 PWL sixteen
-// 21.3 -> 18.1 ms, 112^3 PWC seven 1.38 -> 1.08 ms.  What bounds it: at few
+// of kx in S), ellipsoids that leave 5% of the slices empty: 96^3 PWL one right-hand
+// side 0.814 -> 0.532 ms, 128^3 PWL sixteen 21.3 -> 18.1 ms, 112^3 PWC seven 1.38 ->
+// 1.08 ms.  What bounds it: at few
 // right-hand sides the Green columns were (a quarter of them is read now), then
 // the data path of shared memory and L1 (60-70% busy: 13 thousand clocks a
 // 128^3 PWL tile, 6 of them the product's inputs and Green values) and the FMA
@@ -34,7 +35,9 @@
 //    registers during the last inverse step (a task of step B and the same task
 //    of the next tile's step 1 own the same place in shared memory, so no
 //    barrier stands between them);
-//  * tasks are small enough for 128 registers, sixteen warps an SM;
+//  * tasks are small enough for 128 registers, sixteen warps an SM (a few of them
+//    spill: 8 to 28 bytes a thread at n3 = 64 and more, 20 to 150 at 16 to 48, whose
+//    tasks hold sixteen inputs at once);
 //  * the product gives a thread the outputs of one moment l (of the three
 //    vector components) for two elements that share their Green column, and
 //    loads the Green values of its next input moment while it multiplies by the

@@ -6,15 +6,17 @@
 // right-hand side) in the y passes, so all three transforms read and write runs of W
 // elements (256 bytes at W = 32), and a z-pass column is one contiguous run.  (With
 // rows of kx in T1 and columns of z in S one of the two sides of the y passes had runs
-// of 64 bytes: 128^3 PWL, every slice live, sixteen right-hand sides, 4.4 + 4.5 ms; now
-// 3.5 + 4.1.)
+// of 64 bytes: 128^3 PWL, sixteen right-hand sides, a body in 95% of the slices and half
+// of the rows, 4.4 + 4.5 ms; now 3.5 + 3.5.)
 //
 // Both halves of a zero-padded transform (even and odd frequencies) run in the
 // two lanes of packed FP32 pairs (pair.cuh), one instruction for both, and pass
 // through shared memory as 16-byte pairs: sequence e at e*S, S = 16*NB + 1
 // pairs, [k1][b] (consecutive e on distinct 16-byte bank groups).  128^3 PWL,
 // sixteen right-hand sides, against one half after the other: X 1.86 -> 1.41,
-// YI 4.10 -> 3.58 ms.
+// YI 4.10 -> 3.58 ms (the body above).  A tile is skipped where all of its rows or
+// slices are empty: with 28% of the rows live, X takes 0.97 ms where tiles of one row,
+// both halves in turn, took 0.87.
 #pragma once
 
 #include "matvec4.cuh"
@@ -303,8 +305,8 @@ __device__ __forceinline__ bool y_tile(const MvArgs<float>& a, int& f0, int& z) 
   return any;
 }
 
-// One half at a time in scalar arithmetic at 80 registers: the pass waits for
-// HBM, and three CTAs an SM hold more loads in flight than two of the packed
+// One half at a time in scalar arithmetic at 80 registers (64 bytes a thread spilled):
+// the pass waits for HBM, and three CTAs an SM hold more loads in flight than two of the packed
 // form (48^3 PWL, eight right-hand sides: 139 against 158 us; 128^3: the same).
 template <int NB>
 __global__ void __launch_bounds__(256, 3) k4c_fwd_y(MvArgs<float> a) {
