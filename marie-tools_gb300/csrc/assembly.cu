@@ -455,8 +455,8 @@ static cudaError_t run_vv(const int4* offs, int nspec, int noff, const DevRule* 
 // ---------------------------------------------------------------------------
 
 // Ue[l][comp*Ns + s] = coef of loop l on voxel s; one thread per (voxel, loop).
-// Segments: seg[(l*nseg + i)*6 + {mid xyz, dl xyz}]; dlsum[3l + p]: the sum of a
-// loop's dl.
+// Segments: seg[(l*nseg + i)*6 + {mid xyz, dl xyz}]; whole[7l + {sum of the loop's dl
+// xyz, its centre xyz, mean squared distance of its mid-points from the centre}].
 //
 // Bound by FP64: 27 points (three Gauss points per axis) times nseg segments per
 // voxel, each 1/R and exp(-iR).  So the squares of the coordinate differences are
@@ -464,21 +464,23 @@ static cudaError_t run_vv(const int4* offs, int nspec, int noff, const DevRule* 
 // segment (its dl factors out of the points); and with SMALL (k0 times the distance
 // to the voxel's centre point at most 0.05) the phase is the centre's times that of
 // R - R_centre, a short series.  About thirty FP64 operations a value instead of
-// seventy: 64^3 PWL, four loops of 64 segments, 55.6 -> 32.1 ms.
+// seventy: 64^3 PWL, four loops of 64 segments, 55.6 -> 31.8 ms.
 //
 // Rounding: the dl of a closed loop add up to zero, so the field is a small
-// difference of the segments' values.  The value of the first segment's centre point
-// is subtracted from all of them where they are formed (an FMA in place of a product)
-// and its part of the sum added at the end, with the dl summed on the host: what the
-// sums then round is the difference (error 4.6e-16 of the field at 24^3 PWL, 7.8 mm,
-// where the values themselves give 1.4e-15 and plain FP64 point by point 1.7e-15).
+// difference of the segments' values.  The value at the root mean square distance of
+// the voxel's centre from the loop is subtracted from all of them where they are formed
+// (an FMA in place of a product) and its part of the sum added at the end, with the dl
+// summed on the host: what the sums then round is the difference (error 4.0e-16 of the
+// field at 24^3 PWL, 7.8 mm, where the values themselves give 1.4e-15 and plain FP64
+// point by point 1.7e-15).  That distance is a typical one at every voxel and never
+// small, also where a segment passes through the voxel.
 constexpr int kLoopThreads = 128;
 constexpr int kLoopTile = 64;      // segments staged in shared memory
 
 template <bool PWL, bool SMALL>
 __global__ void __launch_bounds__(kLoopThreads) k_loops(const int64_t* idxS, int64_t Ns, int n1, int n2, double ox,
                                                         double oy, double oz, double res, const double* seg, int nseg,
-                                                        const double* dlsum, const double* qx, const double* qw,
+                                                        const double* whole, const double* qx, const double* qw,
                                                         double k0, double f, zd* out) {
   __shared__ double tile[kLoopTile * 6];
   constexpr int L = PWL ? 4 : 1;
@@ -491,7 +493,7 @@ __global__ void __launch_bounds__(kLoopThreads) k_loops(const int64_t* idxS, int
   double o[3], w[3], v[3];       // point offsets, weights, weights times the linear moment
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    o[a] = 0.5 * res * qx[a];
+    o[a] = 0.5 * res * k0 * qx[a];
     w[a] = 0.5 * qw[a];
     v[a] = w[a] * (0.5 * qx[a]);
   }
@@ -503,9 +505,10 @@ __global__ void __launch_bounds__(kLoopThreads) k_loops(const int64_t* idxS, int
   const double* sg = seg + (int64_t)l * nseg * 6;
   double g0x = 0, g0y = 0;       // cos(R)/R and sin(R)/R subtracted from every value
   if (on) {
-    const double dx = k0 * (cx - sg[0]), dy = k0 * (cy - sg[1]), dz = k0 * (cz - sg[2]);
+    const double* m = whole + 7 * l + 3;
+    const double dx = cx - m[0], dy = cy - m[1], dz = cz - m[2];
     double R, sn, cs;
-    const double iR = inv_sqrt(dx * dx + dy * dy + dz * dz, R);
+    const double iR = inv_sqrt(k0 * k0 * (dx * dx + dy * dy + dz * dz + m[3]), R);
     sin_cos(R, &sn, &cs);
     g0x = cs * iR;
     g0y = sn * iR;
@@ -519,9 +522,12 @@ __global__ void __launch_bounds__(kLoopThreads) k_loops(const int64_t* idxS, int
     for (int i = 0; i < nt; ++i) {
       const double* q = tile + 6 * i;
       double x2[3], y2[3], z2[3];
+      // a point's offset is added to the centre's difference: where a segment is near, the
+      // coordinates' own rounding does not enter
+      const double ex = cx - q[0], ey = cy - q[1], ez = cz - q[2];
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const double dx = k0 * (cx + o[a] - q[0]), dy = k0 * (cy + o[a] - q[1]), dz = k0 * (cz + o[a] - q[2]);
+        const double dx = fma(k0, ex, o[a]), dy = fma(k0, ey, o[a]), dz = fma(k0, ez, o[a]);
         x2[a] = dx * dx;
         y2[a] = dy * dy;
         z2[a] = dz * dz;
@@ -599,8 +605,8 @@ __global__ void __launch_bounds__(kLoopThreads) k_loops(const int64_t* idxS, int
   if (!on) return;
 #pragma unroll
   for (int p = 0; p < 3; ++p) {   // the weights of the constant moment add up to one, of the linear ones to zero
-    acc[p][0].x = fma(dlsum[3 * l + p], g0x, acc[p][0].x);
-    acc[p][0].y = fma(dlsum[3 * l + p], g0y, acc[p][0].y);
+    acc[p][0].x = fma(whole[7 * l + p], g0x, acc[p][0].x);
+    acc[p][0].y = fma(whole[7 * l + p], g0y, acc[p][0].y);
   }
   // E = -i omega mu0 sum exp(-ikR)/(4 pi R) dl, f = omega mu0 k0 / (4 pi)
 #pragma unroll
@@ -763,8 +769,8 @@ extern "C" marie_status marie_incident_loops(marie_vie* h, const double* origin,
     return MARIE_ERR_BAD_ARG;
   }
   // regular nseg-gon inscribed in each circle: mid-points and chord vectors
-  std::vector<double> seg((size_t)nloop * nseg * 6 + 3 * (size_t)nloop);
-  double* const dlsum = seg.data() + (size_t)nloop * nseg * 6;
+  std::vector<double> seg((size_t)nloop * nseg * 6 + 7 * (size_t)nloop);
+  double* const whole = seg.data() + (size_t)nloop * nseg * 6;
   for (int l = 0; l < nloop; ++l) {
     const double* L = loops + 6 * l;
     double nx = L[3], ny = L[4], nz = L[5];
@@ -793,8 +799,11 @@ extern "C" marie_status marie_incident_loops(marie_vie* h, const double* origin,
     for (int p = 0; p < 3; ++p) {
       long double sum = 0;
       for (int i = 0; i < nseg; ++i) sum += seg[((size_t)l * nseg + i) * 6 + 3 + p];
-      dlsum[3 * l + p] = (double)sum;
+      whole[7 * l + p] = (double)sum;
+      whole[7 * l + 3 + p] = L[p];
     }
+    const double rm = radius * std::cos(M_PI / nseg);
+    whole[7 * l + 6] = rm * rm;
   }
   std::vector<void*> scratch;
   auto done = [&](marie_status s) {

@@ -73,3 +73,32 @@ def test_no_worse_than_plain_fp64(res, freq):
     print(rel)
     assert rel["gpu"][0] <= rel["plain"][0] and rel["gpu"][1] <= 2 * rel["plain"][1], rel
     op.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("res,freq", [(2.0 ** -7, 128e6), (2.0 ** -6, 297.2e6)])
+def test_segment_through_a_voxel_centre(res, freq):
+    """The first segment's mid-point 1e-9 voxels from a voxel's centre: the linear
+    moments, in which the centre point has no weight, stay those of plain sums (a few
+    hundred units of 2^-53 of the voxel's largest, for the cancellation of the dl)."""
+    from marie_gb300 import VieOperator, phantoms
+    n, nseg, radius = 16, 64, 2.0 ** -5
+    body = phantoms.sphere(n, res, 0.45 * n * res, 30.0, 0.5)
+    op = VieOperator(body.n, res, freq, body.idx_solution(True), body.Mr(freq), np.zeros((n, n, n, 10, 6), complex), pwl=True,
+                     precisions=2)
+    lin = int(body.idxS[op.Ns // 2])
+    at = body.origin + res * np.array([[lin % n, lin // n % n, lin // (n * n)]], np.float64)
+    e1, e2 = np.array([0.0, 0.0, 1.0]), np.array([0.0, -1.0, 0.0])     # normal +x
+    mid = 0.5 * radius * ((1 + math.cos(2 * math.pi / nseg)) * e1 + math.sin(2 * math.pi / nseg) * e2)
+    L = at[0] - mid + 1e-9 * res * np.array([1.0, 0.0, 0.0])
+    got = op.incident_loops(body.origin, np.concatenate([L, [1.0, 0.0, 0.0]])[None], radius, nseg=nseg).cpu().numpy()
+    got = got.reshape(3, 4, -1)[..., op.Ns // 2]
+    pts = [L + radius * (math.cos(t) * e1 + math.sin(t) * e2) for t in (2 * math.pi * i / nseg for i in range(nseg + 1))]
+    k0 = 2 * math.pi / (299792458.0 / freq)
+    ref = _field(np.longdouble, at, res, [(0.5 * (a + b), b - a) for a, b in zip(pts, pts[1:])], k0,
+                 2 * math.pi * freq * (4e-7 * math.pi))[0]
+    want = np.float64(ref[..., 0]) + 1j * np.float64(ref[..., 1])
+    assert np.isfinite(got).all()
+    err = np.abs(got - want)[:, 1:].max() / np.abs(want[:, 1:]).max()
+    assert err < 1e-13, err
+    op.close()
